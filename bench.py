@@ -214,10 +214,12 @@ def jk_form_of(p):
 
 
 def sym_active(p, form, precision, sym="auto"):
-    """Whether the library runs the streamed form with the exchange symmetry (pairs i <= k against the
-    symmetric half of each density, i < k against the antisymmetric half): on by default in FP64 and,
-    for n > 64, in the tensor-core precisions."""
-    return form == "streamed" and sym != "off" and (precision == "fp64" or p.n > 64)
+    """Whether the library runs the exchange-matrix form with the exchange symmetry (pairs i <= k against
+    the symmetric half of each density, i < k against the antisymmetric half): on by default in FP64 and,
+    for n > 64, in the tensor-core precisions (the stored form: int8 only)."""
+    if form == "eri" and precision not in ("fp64", "ozaki_i8"):
+        return False
+    return form in ("eri", "streamed") and sym != "off" and (precision == "fp64" or p.n > 64)
 
 
 def choose_ipanel(n):
@@ -251,14 +253,17 @@ def jk_flops_per_point(p, form, sym=False, precision="ozaki_i8"):
     eri / streamed:  K = EK (n^2 x n^2, real) times 4 complex density columns: 16 n^4, and the
                      Coulomb term d = B vec P, J = B^T d: 8 L n^2 (the streamed form also
                      regenerates EK once per chunk: jk_regen_flops, counted as executed work)
-    streamed with the exchange symmetry: the pair rows times 8 real columns, 16 (p_le^2 + p_lt^2) with
+    with the exchange symmetry: the pair rows times 8 real columns, 16 (p_le^2 + p_lt^2) with
                      p_le = n(n+1)/2 and p_lt = n(n-1)/2 (about 8 n^4); in the tensor-core forms the
-                     Coulomb d runs over the pairs too: 4 L (p_le + n^2)
+                     Coulomb d runs over the pairs too: 4 L (p_le + n^2); the stored FP64
+                     form runs d and J over them: 8 L p_le
     factorized form: T = V^H X (8 L N^2 M), Q = X T' (8 L N^2 M), GX = sum_L B_L Q_L (8 L n^2 N)"""
     n, N, M, L = p.n, p.N, p.M, p.L
-    if form == "streamed" and sym:
+    if form in ("eri", "streamed") and sym:
         ple, plt = n * (n + 1) / 2, n * (n - 1) / 2
-        coul = 8.0 * L * n * n if precision == "fp64" else 4.0 * L * (ple + n * n)
+        coul = 4.0 * L * (ple + n * n)
+        if precision == "fp64":
+            coul = 8.0 * L * (ple if form == "eri" else n * n)
         return 16.0 * (ple * ple + plt * plt) + coul
     if form in ("eri", "streamed"):
         return 16.0 * n ** 4 + 8.0 * L * n * n

@@ -191,13 +191,16 @@ typedef struct {
                                                  shape, int8 GEMM raster group) and keep the fastest; the table
                                                  is shared by all plans of the process.  Results are bitwise
                                                  those of the untuned plan */
-    int exchange_symmetry;                    /* jk_form 3: 0 = automatic (on where available), 1 = on, 2 = off.
-                                                 On: the exchange uses K(rho^T) = K(rho)^T of real integrals --
-                                                 rows (i <= k) against the symmetric half of each density and
-                                                 rows (i < k) against the antisymmetric half, half the exchange
-                                                 GEMM's work and of its rows' regeneration; the FP64 form and the
-                                                 tensor-core forms with n > 64 (n <= 64 tensor-core plans slice
-                                                 the densities in the fused kernel and run the full rows) */
+    int exchange_symmetry;                    /* exchange-matrix forms (jk_form 1, 3): 0 = automatic (on where
+                                                 available), 1 = on, 2 = off.  On: the exchange uses K(rho^T) =
+                                                 K(rho)^T of real integrals -- rows (i <= k) against the symmetric
+                                                 half of each density and rows (i < k) against the antisymmetric
+                                                 half, half the exchange GEMM's work and of its rows'
+                                                 regeneration.  jk_form 3: the FP64 form and the tensor-core forms
+                                                 with n > 64 (n <= 64 tensor-core plans slice the densities in the
+                                                 fused kernel and run the full rows; 1 is refused there).
+                                                 jk_form 1: the FP64 form and the int8 form with n > 64, for
+                                                 exactly symmetric Cholesky vectors (full rows otherwise) */
 } phf_plan_desc;
 
 int phf_plan_create(const phf_plan_desc *desc, phf_plan **plan);

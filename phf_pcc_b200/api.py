@@ -245,11 +245,11 @@ class Plan:
     J/K, FP64 only); "auto" takes "eri" up to n = 128 and "streamed" above.  ``gradient``:
     "reference" (the reference's bra-side gradient, LocalG) or "exact" (dE/dC* including the
     ket-side term; used by autograd).  ``autotune``: time the launch choices of the plan's GEMM shapes
-    at its first evaluation (bitwise the same results).  ``exchange_symmetry`` (streamed form):
-    "auto" (on where available), True or False -- with it the exchange runs over index pairs i <= k
+    at its first evaluation (bitwise the same results).  ``exchange_symmetry`` (exchange-matrix
+    forms): "auto" (on where available), True or False -- with it the exchange runs over index pairs i <= k
     against the symmetric half of each density and i < k against the antisymmetric half (K(rho^T) =
     K(rho)^T for real integrals): half the exchange GEMM's work.  Available in FP64 and, for n > 64,
-    in the tensor-core precisions."""
+    in the tensor-core precisions (stored form: "ozaki_i8" only, and symmetric Cholesky vectors)."""
 
     def __init__(self, *, ref, ngrid, nci, cmplxconj, ncisp, nocc, r1, r2, rpg, weightsp, weightpg, roota, rootb,
                  rooty, qj, sp, h=None, B=None, hone=None, htwo=None, precision="fp64", slices=0,

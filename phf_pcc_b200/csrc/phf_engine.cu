@@ -277,6 +277,20 @@ int choose_ipanel(int n) {
 }
 }  // namespace
 
+namespace {
+// whether every B_L equals its transpose exactly
+bool cholesky_symmetric(const phf_plan_desc *d) {
+    const size_t n = d->nso / 2;
+    for (int l = 0; l < d->nchol; ++l) {
+        const double *B = d->bvec + n * n * (size_t)l;
+        for (size_t q = 0; q < n; ++q)
+            for (size_t p = 0; p < q; ++p)
+                if (B[p + n * q] != B[q + n * p]) return false;
+    }
+    return true;
+}
+}  // namespace
+
 int plan_create(const phf_plan_desc *d, phf_plan **out) {
     *out = nullptr;
     PHF_TRY(validate(d));
@@ -321,13 +335,18 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
         set_error(PHF_ERR_UNSUPPORTED, "the tensor-core precisions need an exchange-matrix form (jk_form 0, 1 or 3)");
         return PHF_ERR_UNSUPPORTED;
     }
+    // the exchange symmetry (n >= 2): the streamed form in FP64 and in the tensor-core forms whose densities
+    // are sliced apart from the density GEMM (n > 64); the stored form in FP64 and in the int8 form with
+    // n > 64, when the Cholesky vectors are exactly symmetric (K(rho^T) = K(rho)^T holds for any real
+    // vectors, the Coulomb term over pairs l <= j only for symmetric ones).  The full rows do twice the
+    // exchange work: an evaluation takes 9.5 ms with them and 5.7 ms without (FP64, n = 64, 800 points),
+    // 25.0 and 16.1 ms (int8, n = 128, 800 points), 5.3 and 4.4 ms (int8, n = 101, 312 points)
+    const bool sym_slices = p.prec == PHF_PREC_FP64 || !oz_rho_slice_ok(d->nso / 2);
     if (p.streamed) {
         const int n = d->nso / 2;
         p.ek_ipanel = d->exchange_panel > 0 ? std::min(d->exchange_panel, n) : choose_ipanel(n);
         p.ek_npanel = (n + p.ek_ipanel - 1) / p.ek_ipanel;
-        // the exchange symmetry: FP64, and the tensor-core forms whose densities are sliced apart from
-        // the density GEMM (n > 64)
-        const bool sym_ok = n >= 2 && n <= 65535 && (p.prec == PHF_PREC_FP64 || !oz_rho_slice_ok(n));
+        const bool sym_ok = n >= 2 && n <= 65535 && sym_slices;
         if (d->exchange_symmetry == 1 && !sym_ok) {
             set_error(PHF_ERR_UNSUPPORTED, "exchange_symmetry needs the FP64 form or n > 64 (tensor-core forms)");
             return PHF_ERR_UNSUPPORTED;
@@ -344,6 +363,12 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
             p.ek_i0.push_back(n);
             p.ek_npanel = (int)p.ek_i0.size() - 1;
         }
+    } else if (p.eri) {
+        const int n = d->nso / 2;
+        p.ek_sym = n >= 2 && n <= 65535 && sym_slices && d->exchange_symmetry != 2 &&
+                   (p.prec == PHF_PREC_FP64 || p.prec == PHF_PREC_OZAKI_I8) && cholesky_symmetric(d);
+        if (p.ek_sym) p.ek_i0 = {0, n};  // one panel: every row, formed once at plan creation
+        p.ek_npanel = 1;
     }
     p.nl = d->ngrid[0];
     p.ny = d->ngrid[1];
@@ -815,6 +840,35 @@ int build_exchange_matrix(PlanImpl &p) {
         PHF_CUDA(cudaDeviceSynchronize());
         return PHF_OK;
     }
+    if (p.ek_sym) {  // the whole Gram block once, then the symmetric and antisymmetric rows of all pairs
+        const long long kks = (long long)n * (n + 1) / 2, kka = (long long)n * (n - 1) / 2;
+        PHF_TRY(upload_pair_tables(p));
+        double *G = nullptr;
+        PHF_TRY(p.arena.alloc(&G, (size_t)(n2 * n2)));
+        OutView go = vo(reinterpret_cast<zc *>(G), n2, 1);
+        go.real = 1;
+        PHF_TRY(zgemm_strided((int)n2, (int)n2, L, 1, 1, Z1, vd(p.Bst, 1, n2), vd(p.Bst, n2, 1), Z0, go, nullptr, 0));
+        if (p.prec == PHF_PREC_FP64) {
+            PHF_TRY(p.arena.alloc(&p.EK, (size_t)(kks * kks + kka * kka)));
+            PHF_TRY(launch_ek_sym_panel(n, 0, n, 0, p.pairs_le, G, n2, p.EK, p.EK + kks * kks, 0));
+            // the Coulomb term over pairs: B_L[l][j] (2 - delta_lj)
+            PHF_TRY(p.arena.alloc(&p.Bpair, (size_t)(L * kks)));
+            PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, p.Bpair, 0));
+        } else {
+            const long long rs = oz_pad_rows(kks), ra = oz_pad_rows(kka);
+            const size_t bs = oz_slice_bytes(rs, kks, p.slices), ba = oz_slice_bytes(ra, kka, p.slices);
+            PHF_TRY(p.arena.alloc(&p.EKsl, bs + ba));
+            PHF_CUDA(cudaMemset(p.EKsl, 0, bs + ba));
+            PHF_TRY(p.arena.alloc(&p.ea, (size_t)(rs + ra)));
+            PHF_CUDA(cudaMemset(p.ea, 0, (size_t)(rs + ra) * sizeof(int)));
+            PHF_TRY(oz_slice_ek_sym_panel(n, 0, n, 0, p.pairs_le, G, n2, p.slices, rs, p.EKsl, p.ea, ra, p.EKsl + bs,
+                                          p.ea + rs, 0));
+            PHF_TRY(build_coulomb_slices(p));
+        }
+        PHF_CUDA(cudaDeviceSynchronize());
+        p.arena.free_one(G);
+        return PHF_OK;
+    }
     double *EK = nullptr;
     PHF_TRY(p.arena.alloc(&EK, (size_t)(n2 * n2)));
     OutView o = vo(reinterpret_cast<zc *>(EK), n, 1, n2, n2 * n);
@@ -859,16 +913,22 @@ int exchange_streamed_sym(PlanImpl &p, int bc, cudaStream_t st) {
         const int grows = ip * n;
         const long long ts0 = pair_index_le(nn, i0, i0), ta0 = rows_a > 0 ? pair_index_lt(nn, i0, i0 + 1) : 0;
         if (p.prec == PHF_PREC_FP64) {
-            double *EKs = p.EKp, *EKa = p.EKp + rows_s * kks;
+            double *EKs = p.streamed ? p.EKp : p.EK, *EKa = EKs + rows_s * kks;
             double *Kv = reinterpret_cast<double *>(p.Kvec);
             const double *Ki = reinterpret_cast<const double *>(p.Kin);
-            if (p.library_gemm) {
+            if (p.library_gemm && cublasSetStream(reinterpret_cast<cublasHandle_t>(p.cublas), st) !=
+                                      CUBLAS_STATUS_SUCCESS) {
+                set_error(PHF_ERR_CUDA, "cublasSetStream failed");
+                return PHF_ERR_CUDA;
+            }
+            if (!p.streamed) {
+                // the stored rows
+            } else if (p.library_gemm) {
                 cublasHandle_t h = reinterpret_cast<cublasHandle_t>(p.cublas);
                 const double one = 1.0, zero = 0.0;
                 ProfScope prof(st, PROF_JK);
                 // column-major: G^T (gcols x grows) = (columns k >= i0 of B^T) * (rows of B^T)^T
-                if (cublasSetStream(h, st) != CUBLAS_STATUS_SUCCESS ||
-                    cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, (int)gcols, grows, L, &one, p.Bst + (size_t)i0 * n,
+                if (cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, (int)gcols, grows, L, &one, p.Bst + (size_t)i0 * n,
                                 (int)n2, p.Bst + (size_t)i0 * n, (int)n2, &zero, p.Gp, (int)gcols) !=
                         CUBLAS_STATUS_SUCCESS) {
                     set_error(PHF_ERR_CUDA, "cublasDgemm (exchange panel) failed");
@@ -880,7 +940,7 @@ int exchange_streamed_sym(PlanImpl &p, int bc, cudaStream_t st) {
                 PHF_TRY(zgemm_strided(grows, (int)gcols, L, 1, 1, Z1, vd(p.Bst + (size_t)i0 * n, 1, n2),
                                       vd(p.Bst + (size_t)i0 * n, n2, 1), Z0, o, nullptr, st));
             }
-            PHF_TRY(launch_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, EKs, EKa, st));
+            if (p.streamed) PHF_TRY(launch_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, EKs, EKa, st));
             if (p.library_gemm) {
                 cublasHandle_t h = reinterpret_cast<cublasHandle_t>(p.cublas);
                 const double one = 1.0, zero = 0.0;
@@ -903,16 +963,18 @@ int exchange_streamed_sym(PlanImpl &p, int bc, cudaStream_t st) {
                                           vo(p.Kvec + (size_t)(kks + ta0) * 4 * b, 4LL * b, 1), nullptr, st));
             }
         } else {
-            OzEx gx;
-            gx.b_rows_pad = oz_pad_rows(n2);
-            gx.b_row0 = i0 * n;
-            PHF_TRY(oz_gemm_ex(grows, (int)gcols, L, p.slices, p.B2sl, oz_pad_rows(n2), i0 * n, p.eB2, p.B2sl, p.eB2,
-                               p.Gp, gcols, 0, 0, p.ozerr, st, 0, 0, gx));
             const long long rps = oz_pad_rows(rows_s), rpa = oz_pad_rows(std::max<long long>(rows_a, 1));
-            signed char *As = p.EKpsl, *Aa = p.EKpsl + oz_slice_bytes(rps, kks, p.slices);
-            int *es = p.eEKp, *ea = p.eEKp + rps;
-            PHF_TRY(oz_slice_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, p.slices, rps, As, es, rpa, Aa, ea,
-                                          st));
+            signed char *As = p.streamed ? p.EKpsl : p.EKsl, *Aa = As + oz_slice_bytes(rps, kks, p.slices);
+            int *es = p.streamed ? p.eEKp : p.ea, *ea = es + rps;
+            if (p.streamed) {
+                OzEx gx;
+                gx.b_rows_pad = oz_pad_rows(n2);
+                gx.b_row0 = i0 * n;
+                PHF_TRY(oz_gemm_ex(grows, (int)gcols, L, p.slices, p.B2sl, oz_pad_rows(n2), i0 * n, p.eB2, p.B2sl,
+                                   p.eB2, p.Gp, gcols, 0, 0, p.ozerr, st, 0, 0, gx));
+                PHF_TRY(oz_slice_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, p.slices, rps, As, es, rpa, Aa,
+                                              ea, st));
+            }
             OzEx sx;
             sx.gamma_mode = 1;
             sx.g_pairs = p.pairs_le;
@@ -1012,7 +1074,15 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
         PHF_TRY(zgemm_strided(M, M, N, bc, 1, Z1, vz(p.Xs, ld, 1, N), vz(p.bra, 1, N, 0, 0, 1), Z0,
                               vo(p.Rho, M, 1, MM), nullptr, st));
     }
-    if (p.prec == PHF_PREC_FP64) {
+    if (p.prec == PHF_PREC_FP64 && p.Bpair) {
+        // over the pairs l <= j: P's symmetric half is the sum of Kin's aa and bb columns; J at pair rows
+        const int kp = n * (n + 1) / 2;
+        PHF_TRY(launch_gather_kin_sym(n, bc, p.pairs_le, p.Rho, p.Kin, 4LL * b, st, p.Pvec, b));
+        PHF_TRY(zgemm_strided(L, bc, kp, 1, 1, Z1, vd(p.Bpair, kp, 1), vz(p.Pvec, b, 1), Z0, vo(p.dvec, b, 1), nullptr,
+                              st));
+        PHF_TRY(zgemm_strided(kp, bc, L, 1, 1, Z1, vd(p.Bpair, 1, kp), vz(p.dvec, b, 1), Z0, vo(p.Jvec, b, 1), nullptr,
+                              st));
+    } else if (p.prec == PHF_PREC_FP64) {
         PHF_TRY(launch_gather_p(n, bc, p.Rho, p.Pvec, b, st));
         PHF_TRY(zgemm_strided(L, bc, (int)n2, 1, 1, Z1, vd(p.Bst, n2, 1), vz(p.Pvec, b, 1), Z0, vo(p.dvec, b, 1),
                               nullptr, st));
@@ -1064,11 +1134,12 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
     }
     prof_set_class(PROF_JK);
     if (p.prec == PHF_PREC_FP64) {
-        if (p.ek_sym)
-            PHF_TRY(launch_gather_kin_sym(n, bc, p.pairs_le, p.Rho, p.Kin, 4LL * b, st));
-        else
+        if (p.ek_sym) {
+            if (!p.Bpair) PHF_TRY(launch_gather_kin_sym(n, bc, p.pairs_le, p.Rho, p.Kin, 4LL * b, st));
+        } else
+
             PHF_TRY(launch_gather_kin(n, bc, p.Rho, p.Kin, 4LL * b, st));
-        if (p.streamed) {
+        if (p.streamed || p.ek_sym) {
             PHF_TRY(exchange_streamed(p, bc, st));
         } else if (p.library_gemm) {
             // row-major Kvec (n^2 x 8bc reals) = EK (n^2 x n^2) Kin (n^2 x 8bc reals), i.e. column-major
@@ -1089,10 +1160,10 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
         }
         prof_set_class(PROF_GEMM);
         PHF_TRY(launch_assemble_gamma(n, bc, p.Jvec, b, nullptr, 0, 0, p.Kvec, 4LL * b, nullptr, 0, 0, p.Gam, st,
-                                      p.ek_sym, p.fold_h ? p.h : nullptr));
+                                      p.ek_sym ? (p.Bpair ? 2 : 1) : 0, p.fold_h ? p.h : nullptr));
     } else {
         // K (as K^T, 8 bc x n^2) written by the GEMM epilogue as -K into Gamma's complex M x M blocks
-        if (p.streamed)
+        if (p.streamed || p.ek_sym)
             PHF_TRY(exchange_streamed(p, bc, st));
         else
             PHF_TRY(oz_gemm_t((int)n2, 8 * bc, (int)n2, p.slices, p.EKsl, p.ea, p.Bsl, p.eb,

@@ -139,7 +139,9 @@ int launch_assemble_gamma(int n, int b, const zc *J, long long ldj, const double
 // order) followed by its antisymmetric rows (pair_lt order) from the dense densities
 int launch_ek_sym_panel(int n, int i0, int ipanel, int k0, const int *pairs, const double *G, long long ldg,
                         double *EKs, double *EKa, cudaStream_t st);
-int launch_gather_kin_sym(int n, int b, const int *pairs, const zc *rho, zc *Kin, long long ldk, cudaStream_t st);
+// (with P: also P[t ldp + w], the symmetric half of rho^{aa} + rho^{bb} at pair t)
+int launch_gather_kin_sym(int n, int b, const int *pairs, const zc *rho, zc *Kin, long long ldk, cudaStream_t st,
+                          zc *P = nullptr, long long ldp = 0);
 
 // ozaki_i8.cu: FP64-accurate GEMM from int8 slices on tcgen05.  The slice-count argument S is 1..7
 // int8 slices, or one of two floating-point operand formats contracted by the same kernel:
@@ -232,7 +234,7 @@ struct PlanImpl {
                                      // from the Cholesky vectors in panels of ek_ipanel spatial indices i,
                                      // each used against the whole chunk and then overwritten
     int ek_ipanel = 0, ek_npanel = 0;
-    int ek_sym = 0;                  // streamed form with the exchange symmetry (pairs i <= k, i < k)
+    int ek_sym = 0;                  // exchange-matrix form with the exchange symmetry (pairs i <= k, i < k)
     std::vector<int> ek_i0;          // symmetric form: panel p covers indices [ek_i0[p], ek_i0[p + 1])
     int *pairs_le = nullptr, *pairs_lt = nullptr;  // pair t -> i << 16 | k, i <= k, resp. i < k, row order
     int *eb_a = nullptr;             // exponents of the antisymmetric density columns (tensor-core form)
@@ -285,7 +287,10 @@ struct PlanImpl {
     zc *accKG = nullptr, *compKG = nullptr, *accKR = nullptr, *compKR = nullptr, *dummyHS = nullptr;
     long long *offs_k = nullptr;       // 3 x 3 x nomega: GEMM offsets of R1^H, R2^H, Rpg^H per point
     // spatial-ERI exchange form
-    double *EK = nullptr;              // EK[(i n + k) n^2 + l n + j] = (il|kj), FP64 back-end
+    double *EK = nullptr;              // EK[(i n + k) n^2 + l n + j] = (il|kj), FP64 back-end; with the exchange
+                                       // symmetry the symmetric rows (pairs i <= k, l <= j), then the
+                                       // antisymmetric ones
+    double *Bpair = nullptr;           // stored symmetric FP64 form: B_L[l][j] (2 - delta_lj), L x n(n+1)/2
     double *Gp = nullptr;              // streamed form: Gram block of one panel, G[(i - i0) n + l][k n + j]
     double *EKp = nullptr;             // streamed FP64 form: the panel's exchange rows (ipanel n x n^2)
     signed char *EKpsl = nullptr;      // streamed tensor-core form: the panel's exchange rows, sliced

@@ -274,7 +274,8 @@ __global__ void gather_kin_kernel(int n, int b, const zc *rho, zc *Kin, long lon
 // K: complex Kc[(i n + k) ldk + 4 w + st], or pairs with element (ik, c) of Kr at Kr[ik krs + c kcs],
 //    c = 2 (4 w + st) + part.  ksym (complex Kc only): K from its symmetric-form parts, KS of the pair
 //    (min(i, k), max(i, k)) at row pair_le and KA at row n(n + 1)/2 + pair_lt (row order of the pairs),
-//    K[i][k] = KS + KA for i < k, KS - KA for i > k, KS for i = k.
+//    K[i][k] = KS + KA for i < k, KS - KA for i > k, KS for i = k.  ksym 2: J too at pair rows, as
+//    sum_L B_L[i][k] (2 - delta_ik) d_L (so J = J[pair] / 2 off the diagonal).
 __global__ void assemble_gamma_kernel(int n, int b, const zc *J, long long ldj, const double *Jr, long long jrs,
                                       long long jcs, const zc *Kc, long long ldk, const double *Kr, long long krs,
                                       long long kcs, zc *Gam, int ksym, const double *h) {
@@ -291,6 +292,7 @@ __global__ void assemble_gamma_kernel(int n, int b, const zc *J, long long ldj, 
             const long long lo = i < k ? i : k, hi = i < k ? k : i, nn = n;
             const long long ts = lo * nn - lo * (lo - 1) / 2 + (hi - lo);
             kv = Kc[ts * ldk + 4 * w + st];
+            ik = ksym == 2 ? ts : ik;
             if (lo != hi) {
                 const long long ta = nn * (nn + 1) / 2 + lo * (nn - 1) - lo * (lo - 1) / 2 + (hi - lo - 1);
                 const zc ka = Kc[ta * ldk + 4 * w + st];
@@ -304,9 +306,9 @@ __global__ void assemble_gamma_kernel(int n, int b, const zc *J, long long ldj, 
         }
         zc g = mkz(-kv.x, -kv.y);
         if (sg == tu) {
-            if (J) g = g + J[ik * ldj + w];
+            if (J) g = g + (ksym == 2 && i != k ? 0.5 : 1.0) * J[ik * ldj + w];
             else g = g + mkz(Jr[ik * jrs + 2 * w * jcs], Jr[ik * jrs + (2 * w + 1) * jcs]);
-            if (h) g.x += h[ik];
+            if (h) g.x += h[(long long)i * n + k];
         }
         Gam[e] = g;
     }
@@ -430,8 +432,9 @@ __global__ void __launch_bounds__(256) ek_sym_panel_kernel(int n, int i0, int k0
 // Kin in the symmetric exchange form: rows t = pair_le(l, j) (pairs[t] = l << 16 | j) hold
 // rho_s^{st}[l][j] = (rho_w[2l + s][2j + t] + rho_w[2j + s][2l + t]) / 2 at column 4w + st (row stride ldk);
 // rows n(n+1)/2 + pair_lt(l, j), l < j, the antisymmetric halves (difference / 2).  rho_w dense M x M.
+// With P: also P[t ldp + w] = the symmetric half of rho^{aa} + rho^{bb} (the thread of st = 0 adds st = 3's).
 __global__ void gather_kin_sym_kernel(int n, int b, const int *__restrict__ pairs, const zc *rho, zc *Kin,
-                                      long long ldk) {
+                                      long long ldk, zc *P, long long ldp) {
     const int M = 2 * n;
     const long long nn = n, kks = nn * (nn + 1) / 2, tot = kks * b * 4;
     for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < tot; e += (long long)gridDim.x * NT) {
@@ -447,6 +450,11 @@ __global__ void gather_kin_sym_kernel(int n, int b, const int *__restrict__ pair
             Kin[t * ldk + c] = mkz(0.5 * (v.x + u.x), 0.5 * (v.y + u.y));
             const long long ta = kks + (long long)l * (nn - 1) - (long long)l * (l - 1) / 2 + (j - l - 1);
             Kin[ta * ldk + c] = mkz(0.5 * (v.x - u.x), 0.5 * (v.y - u.y));
+        }
+        if (P && (c & 3) == 0) {
+            const zc p = v + R[(long long)(2 * l + 1) * M + 2 * j + 1];
+            const zc q = R[(long long)(2 * j) * M + 2 * l] + R[(long long)(2 * j + 1) * M + 2 * l + 1];
+            P[t * ldp + w] = mkz(0.5 * (p.x + q.x), 0.5 * (p.y + q.y));
         }
     }
 }
@@ -680,9 +688,11 @@ int launch_ek_sym_panel(int n, int i0, int ipanel, int k0, const int *pairs, con
     return PHF_OK;
 }
 
-int launch_gather_kin_sym(int n, int b, const int *pairs, const zc *rho, zc *Kin, long long ldk, cudaStream_t st) {
+int launch_gather_kin_sym(int n, int b, const int *pairs, const zc *rho, zc *Kin, long long ldk, cudaStream_t st,
+                          zc *P, long long ldp) {
     ProfScope prof(st, PROF_MEMORY);
-    gather_kin_sym_kernel<<<grid_for((long long)n * (n + 1) / 2 * b * 4), NT, 0, st>>>(n, b, pairs, rho, Kin, ldk);
+    gather_kin_sym_kernel<<<grid_for((long long)n * (n + 1) / 2 * b * 4), NT, 0, st>>>(n, b, pairs, rho, Kin, ldk, P,
+                                                                                       ldp);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     return PHF_OK;
