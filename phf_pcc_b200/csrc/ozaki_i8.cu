@@ -1101,14 +1101,16 @@ __global__ void __launch_bounds__(SL_NT) slice_rows_kernel(int m, int k, const d
 
 // The same for short rows (kpad <= 1024): one warp per row, eight rows per CTA, the row maximum by
 // warp shuffles (one CTA per row leaves most of a 256-thread block idle when k is a few hundred).
+// Row r is row (r % inner) istride + r / inner of A (inner = 0: row r).
 constexpr int SLW_ROWS = 8;
 __global__ void __launch_bounds__(32 * SLW_ROWS) slice_rows_warp_kernel(int m, int k, const double *A, long long lda,
                                                                         long long cs, int S, long long mpad,
-                                                                        long long kpad, signed char *out, int *ea) {
+                                                                        long long kpad, signed char *out, int *ea,
+                                                                        int inner, long long istride) {
     const long long row = (long long)blockIdx.x * SLW_ROWS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= m) return;
-    const double *a = A + row * lda;
+    const double *a = A + (inner ? (row % inner) * istride + row / inner : row) * lda;
     double mx = 0.0;
     for (int j = lane; j < k; j += 32) mx = fmax(mx, fabs(a[(long long)j * cs]));
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -1571,16 +1573,16 @@ __global__ void __launch_bounds__(SXC_NT) slice_xcols_kernel(int M, int N, const
 }
 
 // Rows of the Cholesky operand of the symmetric Coulomb contraction: row L holds B_L[l][j] (2 - delta_lj)
-// at k-index pair_le(l, j) (B_L[l][j] = Bst[L n^2 + l n + j]), as FP64 rows of length n (n + 1) / 2.
+// (off = 2, or B_L[l][j] with off = 1) at k-index pair_le(l, j) (B_L[l][j] = Bst[L n^2 + l n + j]), as FP64 rows of length n (n + 1) / 2.
 __global__ void cholesky_pairs_kernel(int n, int L, const double *__restrict__ Bst, const int *__restrict__ pairs,
-                                      double *out) {
+                                      double *out, double off) {
     const long long kks = (long long)n * (n + 1) / 2, tot = kks * L, n2 = (long long)n * n;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
          e += (long long)gridDim.x * blockDim.x) {
         const long long row = e / kks, t = e - row * kks;
         const int pr = pairs[t], l = pr >> 16, j = pr & 0xffff;
         const double b = Bst[row * n2 + (long long)l * n + j];
-        out[e] = l == j ? b : 2.0 * b;
+        out[e] = l == j ? b : off * b;
     }
 }
 
@@ -1913,9 +1915,24 @@ int oz_slice_rows_strided(int m, int k, const double *A, long long lda, long lon
     ProfScope prof(st, PROF_MEMORY);
     if (oz_pad_k(k) <= 1024)
         slice_rows_warp_kernel<<<(unsigned)((m + SLW_ROWS - 1) / SLW_ROWS), 32 * SLW_ROWS, 0, st>>>(
-            m, k, A, lda, cs, S, rows_pad, oz_pad_k(k), out, ea);
+            m, k, A, lda, cs, S, rows_pad, oz_pad_k(k), out, ea, 0, 0);
     else
         slice_rows_kernel<<<m, SL_NT, 0, st>>>(m, k, A, lda, cs, S, rows_pad, oz_pad_k(k), out, ea);
+    ++g_launches;
+    PHF_CHECK_LAUNCH();
+    return PHF_OK;
+}
+
+int oz_slice_point_rows(int M, int b, int bc, int k, const double *A, long long lda, int S, long long rows_pad,
+                        signed char *out, int *ea, cudaStream_t st) {
+    const long long m = (long long)M * bc;
+    if (M < 1 || b < bc || m > rows_pad || m > 2147483647LL || !oz_format_ok(S)) {
+        set_error(PHF_ERR_ARG, "oz_slice_point_rows: rows outside the slice buffer");
+        return PHF_ERR_ARG;
+    }
+    ProfScope prof(st, PROF_MEMORY);
+    slice_rows_warp_kernel<<<(unsigned)((m + SLW_ROWS - 1) / SLW_ROWS), 32 * SLW_ROWS, 0, st>>>(
+        (int)m, k, A, lda, 1, S, rows_pad, oz_pad_k(k), out, ea, M, b);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     return PHF_OK;
@@ -2018,9 +2035,9 @@ int oz_slice_xcols(int M, int N, int batch, const zc *X, long long ld, int S, lo
     return PHF_OK;
 }
 
-int oz_cholesky_pairs(int n, int L, const double *Bst, const int *pairs, double *out, cudaStream_t st) {
+int oz_cholesky_pairs(int n, int L, const double *Bst, const int *pairs, double *out, cudaStream_t st, double off) {
     ProfScope prof(st, PROF_MEMORY);
-    cholesky_pairs_kernel<<<148 * 8, 256, 0, st>>>(n, L, Bst, pairs, out);
+    cholesky_pairs_kernel<<<148 * 8, 256, 0, st>>>(n, L, Bst, pairs, out, off);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     return PHF_OK;

@@ -278,14 +278,16 @@ int choose_ipanel(int n) {
 }  // namespace
 
 namespace {
-// whether every B_L equals its transpose exactly
+// whether every B_L equals its transpose exactly (16 x 16 tiles, so that both sides stay in cache)
 bool cholesky_symmetric(const phf_plan_desc *d) {
-    const size_t n = d->nso / 2;
+    const int n = d->nso / 2, T = 16;
     for (int l = 0; l < d->nchol; ++l) {
-        const double *B = d->bvec + n * n * (size_t)l;
-        for (size_t q = 0; q < n; ++q)
-            for (size_t p = 0; p < q; ++p)
-                if (B[p + n * q] != B[q + n * p]) return false;
+        const double *B = d->bvec + (size_t)n * n * l;
+        for (int q0 = 0; q0 < n; q0 += T)
+            for (int p0 = 0; p0 <= q0; p0 += T)
+                for (int q = q0; q < std::min(q0 + T, n); ++q)
+                    for (int p = p0; p < std::min(p0 + T, q); ++p)
+                        if (B[p + (size_t)n * q] != B[q + (size_t)n * p]) return false;
     }
     return true;
 }
@@ -341,6 +343,7 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
     // vectors, the Coulomb term over pairs l <= j only for symmetric ones).  The full rows do twice the
     // exchange work: an evaluation takes 9.5 ms with them and 5.7 ms without (FP64, n = 64, 800 points),
     // 25.0 and 16.1 ms (int8, n = 128, 800 points), 5.3 and 4.4 ms (int8, n = 101, 312 points)
+    const bool symmetric = p.chol && cholesky_symmetric(d);
     const bool sym_slices = p.prec == PHF_PREC_FP64 || !oz_rho_slice_ok(d->nso / 2);
     if (p.streamed) {
         const int n = d->nso / 2;
@@ -365,11 +368,13 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
         }
     } else if (p.eri) {
         const int n = d->nso / 2;
-        p.ek_sym = n >= 2 && n <= 65535 && sym_slices && d->exchange_symmetry != 2 &&
-                   (p.prec == PHF_PREC_FP64 || p.prec == PHF_PREC_OZAKI_I8) && cholesky_symmetric(d);
+        p.ek_sym = n >= 2 && n <= 65535 && (sym_slices || (d->slices == 0 && rz_ok(n, d->nchol))) &&
+                   d->exchange_symmetry != 2 && (p.prec == PHF_PREC_FP64 || p.prec == PHF_PREC_OZAKI_I8) && symmetric;
         if (p.ek_sym) p.ek_i0 = {0, n};  // one panel: every row, formed once at plan creation
         p.ek_npanel = 1;
     }
+    p.rz = p.ek_sym && p.prec == PHF_PREC_OZAKI_I8 && d->slices == 0 && symmetric &&
+           rz_ok(d->nso / 2, d->nchol);
     p.nl = d->ngrid[0];
     p.ny = d->ngrid[1];
     p.npg = d->npg;
@@ -531,17 +536,18 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
     // Hamiltonian
     if (p.chol) {
         const int L = p.L;
-        std::vector<double> hh((size_t)n * n), Bst((size_t)L * n * n);
+        std::vector<double> hh((size_t)n * n), Bst(symmetric ? 0 : (size_t)L * n * n);
         for (int i = 0; i < n; ++i)
             for (int j = 0; j < n; ++j) hh[(size_t)i * n + j] = d->h[(size_t)i + (size_t)n * j];
-        for (int l = 0; l < L; ++l)
+        for (int l = 0; l < L && !symmetric; ++l)  // (symmetric vectors need no transposition)
             for (int pp = 0; pp < n; ++pp)
                 for (int q = 0; q < n; ++q)
                     Bst[((size_t)l * n + pp) * n + q] = d->bvec[(size_t)pp + (size_t)n * ((size_t)q + (size_t)n * l)];
         PHF_TRY(p.arena.alloc(&p.h, hh.size()));
-        PHF_TRY(p.arena.alloc(&p.Bst, Bst.size()));
+        PHF_TRY(p.arena.alloc(&p.Bst, (size_t)L * n * n));
         PHF_CUDA(cudaMemcpy(p.h, hh.data(), hh.size() * sizeof(double), cudaMemcpyHostToDevice));
-        PHF_CUDA(cudaMemcpy(p.Bst, Bst.data(), Bst.size() * sizeof(double), cudaMemcpyHostToDevice));
+        PHF_CUDA(cudaMemcpy(p.Bst, symmetric ? d->bvec : Bst.data(), (size_t)L * n * n * sizeof(double),
+                            cudaMemcpyHostToDevice));
         if (p.eri) PHF_TRY(build_exchange_matrix(p));
         // exchange-matrix forms: with h exactly symmetric (H1 = H1^H), H1 is added to Gamma where J is,
         // so one product gives F X = (H1 + J - K) X and e1 = tr(bra^H H1 X) = sum conj(H1 bra) X
@@ -613,8 +619,11 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
         size_t per = 5 * MN + 3 * (size_t)N * N + 8;
         const size_t n2 = (size_t)n * n;
         if (p.chol && p.eri) {
-            per += 2 * MM + 2 * n2 + p.L;                       // Rho, Gam, Pvec, Jvec, dvec
+            per += MM;                                          // Rho and Gam
+            if (!p.rz) per += 2 * n2 + p.L;                     // Pvec, Jvec, dvec
             if (p.prec == PHF_PREC_FP64) per += 8 * n2;         // Kin, Kvec
+            else if (p.rz) per += (rz_operand_bytes(2 * kRzModuli, 8, n * (n + 1) / 2) + rz_operand_bytes(kRzModuli, 2, n * (n + 1) / 2) +
+                                   2 * rz_operand_bytes(kRzModuli, 2, p.L)) / sizeof(zc) + 1;  // the operands and d
             else per += (8 * (n2 + 64) * oz_slots(p.slices)) / sizeof(zc) + 1  // exchange slices
                         + (2 * n2 + 2 * (size_t)p.L) * oz_slots(p.slices) / sizeof(zc) + 1    // Coulomb slices
                         + p.L + n2;                                                // d^T, J pairs
@@ -668,37 +677,57 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
     PHF_TRY(p.arena.alloc(&p.scal, 2 * (size_t)p.b));
     if (p.chol && p.eri) {
         const size_t n2 = (size_t)n * n, b = (size_t)p.b;
-        PHF_TRY(p.arena.alloc(&p.Rho, b * MM));
         PHF_TRY(p.arena.alloc(&p.Gam, b * MM));
-        PHF_TRY(p.arena.alloc(&p.Pvec, b * n2));
-        PHF_TRY(p.arena.alloc(&p.Jvec, b * n2));
-        PHF_TRY(p.arena.alloc(&p.dvec, b * p.L));
+        p.Rho = p.Gam;  // the densities are gathered into the operands before Gamma is written
+        if (!p.rz) {
+            PHF_TRY(p.arena.alloc(&p.Pvec, b * n2));
+            PHF_TRY(p.arena.alloc(&p.Jvec, b * n2));
+            PHF_TRY(p.arena.alloc(&p.dvec, b * p.L));
+        }
         if (p.prec == PHF_PREC_FP64) {
             PHF_TRY(p.arena.alloc(&p.Kin, 4 * b * n2));
             PHF_TRY(p.arena.alloc(&p.Kvec, 4 * b * n2));
         } else {
-            const long long npadK = oz_pad_cols(8 * (long long)b);
-            size_t bsl = oz_slice_bytes(npadK, (long long)n2, p.slices);
-            if (p.ek_sym) {  // symmetric-half columns (k = n(n+1)/2), then the antisymmetric halves
-                p.bsl_a_off = oz_slice_bytes(npadK, (long long)n * (n + 1) / 2, p.slices);
-                bsl = std::max(bsl, p.bsl_a_off + oz_slice_bytes(npadK, (long long)n * (n - 1) / 2, p.slices));
-                PHF_TRY(p.arena.alloc(&p.eb_a, (size_t)npadK));
+            if (p.rz) {
+                const long long kk = (long long)n * (n + 1) / 2;
+                PHF_TRY(p.arena.alloc(&p.rzK, rz_operand_bytes(2 * kRzModuli, 8LL * b, kk)));
+                PHF_TRY(p.arena.alloc(&p.rzKe, 16 * b));
+                PHF_TRY(p.arena.alloc(&p.rzP, rz_operand_bytes(kRzModuli, 2LL * b, kk)));
+                PHF_TRY(p.arena.alloc(&p.rzPe, 2 * b));
+                PHF_TRY(p.arena.alloc(&p.rzD, rz_operand_bytes(kRzModuli, 2LL * b, p.L)));
+                PHF_TRY(p.arena.alloc(&p.rzDe, 2 * b));
+                // residues of one product: all points, or equal parts of at most 1 GiB (whole 256-row tiles)
+                const size_t tile = rz_product_bytes(2 * kRzModuli, 1, p.rz_rows);
+                const long long groups = (p.b + 31) / 32, cap = std::max<long long>(1, (long long)(((size_t)1 << 30) / tile));
+                const long long parts = (groups + cap - 1) / cap;
+                p.rz_sub = (int)std::min<long long>(p.b, 32 * ((groups + parts - 1) / parts));
+                PHF_TRY(p.arena.alloc(&p.rzC, rz_product_bytes(2 * kRzModuli, 8LL * p.rz_sub, p.rz_rows)));
+                PHF_TRY(p.arena.alloc(&p.rzCJ, std::max(rz_product_bytes(kRzModuli, 2LL * p.rz_sub, p.rz_rows),
+                                                        rz_product_bytes(kRzModuli, 2LL * b, p.L))));
+            } else {
+                const long long npadK = oz_pad_cols(8 * (long long)b);
+                size_t bsl = oz_slice_bytes(npadK, (long long)n2, p.slices);
+                if (p.ek_sym) {  // symmetric-half columns (k = n(n+1)/2), then the antisymmetric halves
+                    p.bsl_a_off = oz_slice_bytes(npadK, (long long)n * (n + 1) / 2, p.slices);
+                    bsl = std::max(bsl, p.bsl_a_off + oz_slice_bytes(npadK, (long long)n * (n - 1) / 2, p.slices));
+                    PHF_TRY(p.arena.alloc(&p.eb_a, (size_t)npadK));
+                }
+                PHF_TRY(p.arena.alloc(&p.Bsl, bsl));
+                PHF_CUDA(cudaMemset(p.Bsl, 0, bsl));
+                PHF_TRY(p.arena.alloc(&p.eb, (size_t)npadK));
+                const long long c2 = oz_pad_cols(2 * (long long)b);
+                const size_t psl = oz_slice_bytes(c2, (long long)n2, p.slices);
+                const size_t dsl = oz_slice_bytes(c2, p.L, p.slices);
+                PHF_TRY(p.arena.alloc(&p.Psl, psl));
+                PHF_TRY(p.arena.alloc(&p.dsl, dsl));
+                PHF_CUDA(cudaMemset(p.Psl, 0, psl));
+                PHF_CUDA(cudaMemset(p.dsl, 0, dsl));
+                PHF_TRY(p.arena.alloc(&p.ePc, (size_t)c2));
+                PHF_TRY(p.arena.alloc(&p.edc, (size_t)c2));
+                PHF_TRY(p.arena.alloc(&p.dT, 2 * b * (size_t)p.L));
+                PHF_TRY(p.arena.alloc(&p.dpart, (size_t)kDSplit * 2 * b * (size_t)p.L));
+                PHF_TRY(p.arena.alloc(&p.Jr, 2 * b * n2));
             }
-            PHF_TRY(p.arena.alloc(&p.Bsl, bsl));
-            PHF_CUDA(cudaMemset(p.Bsl, 0, bsl));
-            PHF_TRY(p.arena.alloc(&p.eb, (size_t)npadK));
-            const long long c2 = oz_pad_cols(2 * (long long)b);
-            const size_t psl = oz_slice_bytes(c2, (long long)n2, p.slices);
-            const size_t dsl = oz_slice_bytes(c2, p.L, p.slices);
-            PHF_TRY(p.arena.alloc(&p.Psl, psl));
-            PHF_TRY(p.arena.alloc(&p.dsl, dsl));
-            PHF_CUDA(cudaMemset(p.Psl, 0, psl));
-            PHF_CUDA(cudaMemset(p.dsl, 0, dsl));
-            PHF_TRY(p.arena.alloc(&p.ePc, (size_t)c2));
-            PHF_TRY(p.arena.alloc(&p.edc, (size_t)c2));
-            PHF_TRY(p.arena.alloc(&p.dT, 2 * b * (size_t)p.L));
-            PHF_TRY(p.arena.alloc(&p.dpart, (size_t)kDSplit * 2 * b * (size_t)p.L));
-            PHF_TRY(p.arena.alloc(&p.Jr, 2 * b * n2));
             // n > 64 with int8 slices: rho_w = X_w bra^H for the whole chunk as one int8 GEMM
             p.rho_i8 = !oz_rho_slice_ok(n) && p.slices <= 7;
             if (p.rho_i8) {
@@ -755,25 +784,41 @@ namespace {
 // the symmetric half of P.
 int build_coulomb_slices(PlanImpl &p) {
     const int n = p.n, L = p.L;
+    if (p.rz) {  // residues over the pairs: B_L (2 - delta) (rows L) and B_L[pair] (rows pair)
+        const long long kk = (long long)n * (n + 1) / 2;
+        PHF_TRY(p.arena.alloc(&p.rzB1, rz_operand_bytes(kRzModuli, L, kk)));
+        PHF_TRY(p.arena.alloc(&p.rzB1e, (size_t)L));
+        PHF_TRY(p.arena.alloc(&p.rzB2, rz_operand_bytes(kRzModuli, kk, L)));
+        PHF_TRY(p.arena.alloc(&p.rzB2e, (size_t)kk));
+        double *Bp = nullptr;
+        PHF_TRY(p.arena.alloc(&Bp, (size_t)(L * kk)));
+        PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, Bp, 0, 2.0));
+        PHF_TRY(rz_rows(L, (int)kk, Bp, kk, 1, p.rzB1, p.rzB1e, 0));
+        PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, Bp, 0, 1.0));
+        PHF_TRY(rz_rows(kk, L, Bp, 1, kk, p.rzB2, p.rzB2e, 0));
+        PHF_CUDA(cudaDeviceSynchronize());
+        p.arena.free_one(Bp);
+        if (!p.streamed) return PHF_OK;
+    }
     const long long n2 = (long long)n * n, kc = p.ek_sym ? (long long)n * (n + 1) / 2 : n2;
-    PHF_TRY(p.arena.alloc(&p.ozerr, 1));
-    PHF_CUDA(cudaMemset(p.ozerr, 0, sizeof(int)));
     const size_t b1 = oz_slice_bytes(oz_pad_rows(L), kc, p.slices);
     const size_t b2 = oz_slice_bytes(oz_pad_rows(n2), L, p.slices);
-    PHF_TRY(p.arena.alloc(&p.B1sl, b1));
     PHF_TRY(p.arena.alloc(&p.B2sl, b2));
-    PHF_CUDA(cudaMemset(p.B1sl, 0, b1));
     PHF_CUDA(cudaMemset(p.B2sl, 0, b2));
-    PHF_TRY(p.arena.alloc(&p.eB1, (size_t)oz_pad_rows(L)));
     PHF_TRY(p.arena.alloc(&p.eB2, (size_t)oz_pad_rows(n2)));
-    if (p.ek_sym) {
+    if (!p.rz) {
+        PHF_TRY(p.arena.alloc(&p.B1sl, b1));
+        PHF_CUDA(cudaMemset(p.B1sl, 0, b1));
+        PHF_TRY(p.arena.alloc(&p.eB1, (size_t)oz_pad_rows(L)));
+    }
+    if (p.ek_sym && !p.rz) {
         double *Bp = nullptr;
         PHF_TRY(p.arena.alloc(&Bp, (size_t)(L * kc)));
         PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, Bp, 0));
         PHF_TRY(oz_slice_rows_strided(L, (int)kc, Bp, kc, 1, p.slices, oz_pad_rows(L), p.B1sl, p.eB1, 0));
         PHF_CUDA(cudaDeviceSynchronize());
         p.arena.free_one(Bp);
-    } else {
+    } else if (!p.rz) {
         PHF_TRY(oz_slice_rows_strided(L, (int)n2, p.Bst, n2, 1, p.slices, oz_pad_rows(L), p.B1sl, p.eB1, 0));
     }
     PHF_TRY(oz_slice_rows_strided((int)n2, L, p.Bst, 1, n2, p.slices, oz_pad_rows(n2), p.B2sl, p.eB2, 0));
@@ -808,6 +853,10 @@ int upload_pair_tables(PlanImpl &p) {
 int build_exchange_matrix(PlanImpl &p) {
     const int n = p.n, L = p.L;
     const long long n2 = (long long)n * n;
+    if (p.prec != PHF_PREC_FP64) {
+        PHF_TRY(p.arena.alloc(&p.ozerr, 1));
+        PHF_CUDA(cudaMemset(p.ozerr, 0, sizeof(int)));
+    }
     if (p.streamed) {  // buffers of one exchange panel; the rows themselves are formed per chunk
         // (symmetric form: a panel's Gram block, ip n x (n - i0) n, and its rows, rows_s x n(n+1)/2 plus
         // rows_a x n(n-1)/2 with rows_a < rows_s <= ip (n - i0), fit in the full form's ek_ipanel n x n^2)
@@ -831,10 +880,18 @@ int build_exchange_matrix(PlanImpl &p) {
                     erows = std::max(erows, rs + ra);
                 }
             }
-            PHF_TRY(p.arena.alloc(&p.EKpsl, bytes));
-            PHF_CUDA(cudaMemset(p.EKpsl, 0, bytes));
-            PHF_TRY(p.arena.alloc(&p.eEKp, (size_t)erows));
-            PHF_CUDA(cudaMemset(p.eEKp, 0, (size_t)erows * sizeof(int)));
+            if (p.rz) {
+                const long long kks = (long long)n * (n + 1) / 2;
+                for (int pi = 0; pi < p.ek_npanel; ++pi)
+                    p.rz_rows = std::max(p.rz_rows, sym_rows(n, p.ek_i0[pi], p.ek_i0[pi + 1] - p.ek_i0[pi]));
+                PHF_TRY(p.arena.alloc(&p.rzE, rz_operand_bytes(2 * kRzModuli, p.rz_rows, kks)));
+                PHF_TRY(p.arena.alloc(&p.rzEe, (size_t)(2 * p.rz_rows)));
+            } else {
+                PHF_TRY(p.arena.alloc(&p.EKpsl, bytes));
+                PHF_CUDA(cudaMemset(p.EKpsl, 0, bytes));
+                PHF_TRY(p.arena.alloc(&p.eEKp, (size_t)erows));
+                PHF_CUDA(cudaMemset(p.eEKp, 0, (size_t)erows * sizeof(int)));
+            }
             PHF_TRY(build_coulomb_slices(p));
         }
         PHF_CUDA(cudaDeviceSynchronize());
@@ -854,6 +911,12 @@ int build_exchange_matrix(PlanImpl &p) {
             // the Coulomb term over pairs: B_L[l][j] (2 - delta_lj)
             PHF_TRY(p.arena.alloc(&p.Bpair, (size_t)(L * kks)));
             PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, p.Bpair, 0));
+        } else if (p.rz) {
+            p.rz_rows = kks;
+            PHF_TRY(p.arena.alloc(&p.rzE, rz_operand_bytes(2 * kRzModuli, kks, kks)));
+            PHF_TRY(p.arena.alloc(&p.rzEe, (size_t)(2 * kks)));
+            PHF_TRY(rz_exchange_rows(n, 0, n, 0, p.pairs_le, G, n2, kks, p.rzE, p.rzEe, 0));
+            PHF_TRY(build_coulomb_slices(p));
         } else {
             const long long rs = oz_pad_rows(kks), ra = oz_pad_rows(kka);
             const size_t bs = oz_slice_bytes(rs, kks, p.slices), ba = oz_slice_bytes(ra, kka, p.slices);
@@ -972,8 +1035,41 @@ int exchange_streamed_sym(PlanImpl &p, int bc, cudaStream_t st) {
                 gx.b_row0 = i0 * n;
                 PHF_TRY(oz_gemm_ex(grows, (int)gcols, L, p.slices, p.B2sl, oz_pad_rows(n2), i0 * n, p.eB2, p.B2sl,
                                    p.eB2, p.Gp, gcols, 0, 0, p.ozerr, st, 0, 0, gx));
-                PHF_TRY(oz_slice_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, p.slices, rps, As, es, rpa, Aa,
-                                              ea, st));
+                if (p.rz)
+                    PHF_TRY(rz_exchange_rows(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, p.rz_rows, p.rzE, p.rzEe, st));
+                else
+                    PHF_TRY(oz_slice_ek_sym_panel(n, i0, ip, i0, p.pairs_le, p.Gp, gcols, p.slices, rps, As, es, rpa,
+                                                  Aa, ea, st));
+            }
+            if (p.rz) {
+                RzFock f;
+                f.n = n;
+                f.L = L;
+                f.rows = (int)rows_s;
+                f.pair0 = (int)ts0;
+                f.pairs = p.pairs_le;
+                f.K = p.rzK;
+                f.ek = p.rzKe;
+                f.k_rows = 8LL * b;
+                f.E = p.rzE;
+                f.ee = p.rzEe;
+                f.e_rows = p.rz_rows;
+                f.D = p.rzD;
+                f.ed = p.rzDe;
+                f.d_rows = 2LL * b;
+                f.B2 = p.rzB2;
+                f.e2 = p.rzB2e;
+                f.C = p.rzC;
+                f.CJ = p.rzCJ;
+                f.h = p.fold_h ? p.h : nullptr;
+                f.err = p.ozerr;
+                for (int s0 = 0; s0 < bc; s0 += p.rz_sub) {
+                    f.w0 = s0;
+                    f.pts = std::min(p.rz_sub, bc - s0);
+                    f.Gam = p.Gam + (size_t)s0 * p.M * p.M;
+                    PHF_TRY(rz_fock(f, st));
+                }
+                continue;
             }
             OzEx sx;
             sx.gamma_mode = 1;
@@ -1053,23 +1149,22 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
     const int M = p.M, N = p.N, n = p.n, L = p.L, b = p.b;
     const long long ld = (long long)b * N, MM = (long long)M * M, n2 = (long long)n * n;
     // tensor-core path with n <= 64: the operand columns are formed and sliced in one kernel, no density in HBM
-    const bool fused = p.prec != PHF_PREC_FP64 && oz_rho_slice_ok(n);
-    // n > 64 with int8 slices: the densities of the whole chunk as ONE int8 GEMM.  Row (i, w) of X,
-    // X_w[i][:] at Xs + (i b + w) N (the points' X blocks side by side), is a row of 2N reals
-    // (re, im interleaved), and rho_w[i][j] = sum_k X_w[i][k] conj(bra[j][k]) is its product with
-    // rows 2j (real part) and 2j + 1 (imaginary part) of the bra's 2M x 2N operand.  The result,
-    // (M b) x 2M reals, is rho_w[i][j] at Rho + (i b + w) M + j: row stride b M, point stride M.
-    long long rrs = M, rws = MM;
+    const bool fused = p.prec != PHF_PREC_FP64 && oz_rho_slice_ok(n) && !p.rz;
+    // n > 64 with int8 slices: the densities of the whole chunk as ONE int8 GEMM.  Row (w, i) of X,
+    // X_w[i][:] at Xs + (i b + w) N, is a row of 2N reals (re, im interleaved), and rho_w[i][j] =
+    // sum_k X_w[i][k] conj(bra[j][k]) is its product with rows 2j (real part) and 2j + 1 (imaginary
+    // part) of the bra's 2M x 2N operand: the (M bc) x 2M reals are the points' densities one after
+    // another (rows (i, w) put a point's rows 15 MB apart at n = 200, and the operand kernels, which read
+    // them along both indices, slowed down: 2.0 against 1.7 ms for 608 points)
+    const long long rrs = M, rws = MM;
     if (p.rho_i8) {
         const long long xrows = oz_pad_rows((long long)M * b);
-        PHF_TRY(oz_slice_rows((int)((long long)M * b), 2 * N, reinterpret_cast<const double *>(p.Xs), 2LL * N,
-                              p.slices, xrows, p.Xsl, p.eX, st));
+        PHF_TRY(oz_slice_point_rows(M, b, bc, 2 * N, reinterpret_cast<const double *>(p.Xs), 2LL * N, p.slices, xrows,
+                                    p.Xsl, p.eX, st));
         PHF_TRY(launch_bra_rho_operand(M, N, p.bra, p.BRop, st));
         PHF_TRY(oz_slice_rows(2 * M, 2 * N, p.BRop, 2LL * N, p.slices, oz_pad_cols(2LL * M), p.BRsl, p.eBR, st));
-        PHF_TRY(oz_gemm_t((int)((long long)M * b), 2 * M, 2 * N, p.slices, p.Xsl, p.eX, p.BRsl, p.eBR,
-                          reinterpret_cast<double *>(p.Rho), 2LL * M, 0, 0, p.ozerr, st));
-        rrs = (long long)b * M;
-        rws = M;
+        PHF_TRY(oz_gemm_ex((int)((long long)M * bc), 2 * M, 2 * N, p.slices, p.Xsl, xrows, 0, p.eX, p.BRsl, p.eBR,
+                           reinterpret_cast<double *>(p.Rho), 2LL * M, 0, 0, p.ozerr, st, 0, 0));
     } else if (!fused) {
         PHF_TRY(zgemm_strided(M, M, N, bc, 1, Z1, vz(p.Xs, ld, 1, N), vz(p.bra, 1, N, 0, 0, 1), Z0,
                               vo(p.Rho, M, 1, MM), nullptr, st));
@@ -1091,7 +1186,10 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
     } else {
         if (fused)
             PHF_TRY(oz_rho_slice(n, N, bc, p.Xs, ld, p.bra, p.slices, p.Bsl, p.eb, p.Psl, p.ePc, st));
-        else if (p.ek_sym)
+        else if (p.rz) {
+            PHF_TRY(rz_density(n, bc, p.pairs_le, p.Rho, rrs, rws, 8LL * b, p.rzK, p.rzKe, 2LL * b, p.rzP, p.rzPe, st));
+            PHF_TRY(rz_coulomb_d(n, L, bc, p.rzP, 2LL * b, p.rzPe, p.rzB1, p.rzB1e, p.rzCJ, p.rzD, p.rzDe, p.ozerr, st));
+        } else if (p.ek_sym)
             PHF_TRY(oz_slice_density_sym(n, bc, p.pairs_le, p.Rho, rrs, rws, p.slices, p.Bsl, p.eb,
                                          p.Bsl + p.bsl_a_off, p.eb_a, oz_pad_cols(8LL * bc), p.Psl, p.ePc,
                                          oz_pad_cols(2LL * bc), st));
@@ -1104,9 +1202,9 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
     // wave leaves idle).  Joined before J is added to Gamma.  Not while per-launch profiling is on:
     // event times of overlapping kernels would count the shared time twice.
     cudaStream_t js = st;
-    const bool fork = p.prec != PHF_PREC_FP64 && !g_prof.on;
+    const bool fork = p.prec != PHF_PREC_FP64 && !p.rz && !g_prof.on;
     const int kcoul = p.ek_sym ? n * (n + 1) / 2 : (int)n2;  // Coulomb contraction over pairs l <= j, or all (l, j)
-    if (p.prec != PHF_PREC_FP64 && !fork) {
+    if (p.prec != PHF_PREC_FP64 && !p.rz && !fork) {
         PHF_TRY(oz_gemm_splitk(L, 2 * bc, kcoul, p.slices, p.B1sl, p.eB1, p.Psl, p.ePc, p.dT, L, 1, kDSplit, p.dpart,
                                p.ozerr, st));
         PHF_TRY(oz_slice_rows_strided(2 * bc, L, p.dT, L, 1, p.slices, oz_pad_cols(2LL * bc), p.dsl, p.edc, st));
@@ -1170,7 +1268,8 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
                               reinterpret_cast<double *>(p.Gam), 0, 0, 0, p.ozerr, st, n));
         if (fork) PHF_CUDA(cudaStreamWaitEvent(st, p.ev_join, 0));  // the Coulomb chain is done
         prof_set_class(PROF_GEMM);
-        PHF_TRY(launch_add_coulomb_diag(n, bc, p.Jr, 1, n2, p.Gam, st, p.fold_h ? p.h : nullptr));
+        // (the residue form's J is in Gamma already)
+        if (!p.rz) PHF_TRY(launch_add_coulomb_diag(n, bc, p.Jr, 1, n2, p.Gam, st, p.fold_h ? p.h : nullptr));
     }
     if (p.fx_i8) {
         // F_w X_w for the chunk's points on the int8 path, sub-batch by sub-batch
@@ -1881,7 +1980,7 @@ int plan_eval_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc 
         const int f = bg.h_flags[2 * i], oz = bg.h_flags[2 * i + 1];
         if (oz) {
             set_error(PHF_ERR_CUDA, "phf_eval_batch: instance " + std::to_string(i) +
-                                        ": tensor-core GEMM pipeline wait timed out");
+                                        ": tensor-core GEMM pipeline wait timed out (code " + std::to_string(oz) + ")");
             return PHF_ERR_CUDA;
         }
         if (f & 1) {

@@ -161,6 +161,9 @@ int oz_slice_rows(int m, int k, const double *A, long long lda, int S, long long
                   cudaStream_t st);
 int oz_slice_rows_strided(int m, int k, const double *A, long long lda, long long cs, int S, long long rows_pad,
                           signed char *out, int *ea, cudaStream_t st);
+// rows i b + w of A (i < M, w < bc) in the order w M + i
+int oz_slice_point_rows(int M, int b, int bc, int k, const double *A, long long lda, int S, long long rows_pad,
+                        signed char *out, int *ea, cudaStream_t st);
 // Exchange columns (8 per point) and Coulomb columns (2 per point) of points 0 .. bc-1 of the densities
 // rho_w (element [r][q] of point w at rho[w ws + r rs + q]; rs, ws even), sliced with their exponents.
 int oz_slice_density(int n, int bc, const zc *rho, long long rs, long long ws, int S, signed char *Ksl, int *eK,
@@ -214,14 +217,47 @@ int oz_slice_ek_sym_panel(int n, int i0, int ipanel, int k0, const int *pairs, c
 int oz_slice_density_sym(int n, int bc, const int *pairs, const zc *rho, long long rs, long long ws, int S,
                          signed char *Ks, int *eKs, signed char *Ka, int *eKa, long long npadK, signed char *Psl,
                          int *eP, long long npadP, cudaStream_t st);
-// out (L x n(n+1)/2, FP64): B_L[l][j] (2 - delta_lj) at k-index pair_le(l, j), the Cholesky operand of the
-// symmetric Coulomb contraction
-int oz_cholesky_pairs(int n, int L, const double *Bst, const int *pairs, double *out, cudaStream_t st);
+// out (L x n(n+1)/2, FP64): B_L[l][j] (times `off` for l != j) at k-index pair_le(l, j); off = 2: the Cholesky
+// operand of the symmetric Coulomb contraction
+int oz_cholesky_pairs(int n, int L, const double *Bst, const int *pairs, double *out, cudaStream_t st, double off = 2.0);
 int oz_gemm_splitk(int m, int n, int k, int S, const signed char *Asl, const int *ea, const signed char *Bsl,
                    const int *eb, double *D, long long ldd, int trans, int nsplit, double *part, int *err,
                    cudaStream_t st);
 int oz_gemm(int m, int n, int k, int S, const signed char *Asl, const int *ea, const signed char *Bsl, const int *eb,
             double *D, long long ldd, int accumulate, int *err, cudaStream_t st);
+
+// residue_i8.cu: the symmetric exchange and Coulomb products from residues modulo eleven 8-bit moduli on tcgen05
+// (rows and contraction over the pairs l <= j; n(n+1)/2 and L at most 65536).  Operands: planes x rows x padded k
+// bytes; scale exponents one per row (exchange operands: 2 x rows, parity-major).
+constexpr int kRzModuli = 11;
+bool rz_ok(int n, int L);
+size_t rz_operand_bytes(int planes, long long rows, long long k);          // planes: 2 kRzModuli for the exchange, else kRzModuli
+size_t rz_product_bytes(int planes, long long a_rows, long long b_rows);   // residues of a product
+// density operands of points 0 .. bc - 1: exchange rows 8 w + 4 s + 2 t + part, Coulomb rows 2 w + part
+int rz_density(int n, int bc, const int *pairs, const zc *rho, long long rs, long long ws, long long rows_k,
+               signed char *outk, int *ek, long long rows_p, signed char *outp, int *ep, cudaStream_t st);
+// rows of a real matrix (row r, element j at A[r lda + j cs]) as a right-hand operand
+int rz_rows(long long rows, int k, const double *A, long long lda, long long cs, signed char *out, int *es,
+            cudaStream_t st);
+// exchange rows of a panel (as oz_slice_ek_sym_panel) as a right-hand operand, row = pair of the panel
+int rz_exchange_rows(int n, int i0, int ipanel, int k0, const int *pairs, const double *G, long long ldg,
+                     long long rows_pad, signed char *out, int *es, cudaStream_t st);
+// d = B1 P of bc points as a left-hand operand D (rows_p rows); C: rz_product_bytes(kRzModuli, 2 bc, L) of scratch
+int rz_coulomb_d(int n, int L, int bc, const signed char *P, long long rows_p, const int *ep, const signed char *B1,
+                 const int *e1, unsigned char *C, signed char *D, int *ed, int *err, cudaStream_t st);
+// J (+ h) - K of pairs [pair0, pair0 + rows) and points [w0, w0 + pts) into Gam (Gam at point w0)
+struct RzFock {
+    int n, L, pts, w0, rows, pair0;
+    const int *pairs;                                              // the whole pair table
+    const signed char *K, *E, *D, *B2;                             // density, exchange rows, d, Cholesky pairs
+    long long k_rows, e_rows, d_rows;
+    const int *ek, *ee, *ed, *e2;
+    unsigned char *C, *CJ;                                         // rz_product_bytes of (2 kRzModuli, 8 pts, rows), (kRzModuli, 2 pts, rows)
+    const double *h;                                               // added to J when given
+    zc *Gam;
+    int *err;
+};
+int rz_fock(const RzFock &f, cudaStream_t st);
 
 // Everything a plan owns: sizes, grid tables, Hamiltonian and the chunk workspace.
 struct PlanImpl {
@@ -239,6 +275,16 @@ struct PlanImpl {
     int *pairs_le = nullptr, *pairs_lt = nullptr;  // pair t -> i << 16 | k, i <= k, resp. i < k, row order
     int *eb_a = nullptr;             // exponents of the antisymmetric density columns (tensor-core form)
     size_t bsl_a_off = 0;            // byte offset of their slices in Bsl
+    bool rz = false;                 // its tensor-core GEMM from residues (int8 plans with the default slices)
+    int rz_sub = 0;                  // points per product of the residue scratch
+    long long rz_rows = 0;           // rows of the exchange operand (the largest panel's pairs)
+    signed char *rzK = nullptr, *rzE = nullptr;  // density and exchange operands, their exponents
+    int *rzKe = nullptr, *rzEe = nullptr;
+    signed char *rzP = nullptr, *rzD = nullptr;  // Coulomb: spin-summed densities and d
+    int *rzPe = nullptr, *rzDe = nullptr;
+    signed char *rzB1 = nullptr, *rzB2 = nullptr;  // B_L (2 - delta) over pairs, and its transpose B_L[pair]
+    int *rzB1e = nullptr, *rzB2e = nullptr;
+    unsigned char *rzC = nullptr, *rzCJ = nullptr;  // residues of one product
     int exact = 0;                   // also accumulate the ket-side gradient (gradient_mode 1)
     int library_gemm = 0;            // FP64 exchange GEMM through cuBLAS (comparison form)
     void *cublas = nullptr;          // cublasHandle_t when library_gemm

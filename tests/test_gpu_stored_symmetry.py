@@ -2,7 +2,13 @@
 index pairs against the full rows, at n = 2 (one antisymmetric pair), odd n, a full 64-row FP64 tile, and
 n = 65 (the smallest tensor-core case), one and several chunks.  Cholesky vectors that are not symmetric keep
 the full rows.  Tolerances: FP64 sums of at most n^2 + L terms in another order (1e-12 of the largest
-element); int8 slices 1e-9, the digit remainder of S = 5 with k = n^2."""
+element); int8 slices 1e-9, the digit remainder of S = 5 with k = n^2.
+
+The int8 plans' residue products (n(n+1)/2 pairs as rows and contraction, tiles of 256 x 256, k-steps of 32)
+against the FP64 plan at n <= 64, where every other step is FP64: sizes on both sides of a tile and of a k-step
+(n = 22, 23: 253, 276 pairs; n = 63, 64: 2016 = 63 k-steps, 2080), an odd and a single tile of points, and
+vectors whose squares vanish in FP64.  Tolerance 1e-10: 2^-43.5 sqrt(k) per entry is 4e-12, and sums over
+points amplify an entry's error by less than ten here."""
 import numpy as np
 import pytest
 import torch
@@ -40,3 +46,18 @@ def test_vectors_that_are_not_symmetric_keep_the_full_rows():
     B = p.B + np.random.default_rng(0).normal(scale=0.02, size=p.B.shape)
     for x, y in zip(_sums(p, B=B), _sums(p, B=B, exchange_symmetry=False)):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,N,ngrid,pg,scale,gradient", [
+    (2, 1, (6, 1), "None", 1.0, "reference"), (3, 2, (6, 3), "None", 1.0, "exact"), (22, 7, (6, 4), "None", 1.0, "reference"),
+    (23, 9, (14, 5), "C2v", 1.0, "reference"), (40, 32, (6, 2), "C2v", 1.0, "exact"), (63, 11, (6, 1), "None", 1.0, "reference"),
+    (64, 32, (6, 6), "None", 1.0, "reference"), (12, 5, (6, 3), "None", 1e-80, "reference")])
+def test_residue_products_match_fp64(n, N, ngrid, pg, scale, gradient):
+    p = synth.make_problem(n, N, 4 * n + 1, ngrid=ngrid, seed=n, pg=pg)
+    if scale != 1.0:
+        p.h[:] = 0.0
+        p.B[:] *= scale
+    got, ref = _sums(p, precision="ozaki_i8", gradient=gradient), _sums(p, precision="fp64", gradient=gradient)
+    assert np.abs(got[0][:, 1] - ref[0][:, 1]).max() <= 1e-12 * np.abs(ref[0][:, 1]).max()
+    for x, y in ((got[0][:, 0], ref[0][:, 0]), (got[1], ref[1])):
+        assert np.isfinite(x).all() and np.abs(x - y).max() <= 1e-10 * np.abs(y).max()
