@@ -8,10 +8,13 @@
 //
 // Tiling: BM x BN output tile per CTA of (BM / 32) (BN / 16) warps (64 x 64, 128 x 32 and 32 x 128 on
 // 8 warps; 32 x 112 on 7 and 64 x 112 on 14 for products with 97..112 output columns, such as the
-// per-point products with N = 100 orbitals), k-step 16, the k-tiles staged by cp.async.
-// The products run on the FP64 tensor cores (mma.sync m8n8k4 .f64): each of the 8 warps owns a
-// 32 x 16 block of the tile as 4 x 2 blocks of 8 x 8, and a complex product is four real MMAs
-// (re re, -im im, re im, im re), two for a real A.
+// per-point products with N = 100 orbitals; 32 x 32 on 2 for small products), k-step 16, the k-tiles
+// staged by cp.async.
+// The products run on the FP64 tensor cores (mma.sync m8n8k4 .f64; the larger shapes reach the same 37 TFLOP/s
+// in isolation): each warp owns a 32 x 16 block of the tile as 4 x 2 blocks of 8 x 8, and a complex product
+// is four real MMAs (re re, -im im, re im, im re), two for a real A.  Bound: the FP64 tensor pipe for long k
+// (real 2080 x 2080 by complex 2080 x 3200: 2.19 -> 1.80 ms, 30.8 TFLOP/s, when the address arithmetic left
+// the k loop), latency for the small products (n = 20, 112 points: GEMMs 230 -> 145 us of an evaluation).
 #include <type_traits>
 
 #include "phf_internal.h"
@@ -25,23 +28,20 @@ constexpr int BK = 16;
 template <int BM, int BN>
 __host__ __device__ constexpr int zg_threads() { return (BM / 32) * (BN / 16) * 32; }
 template <int BM, int BN>
-__host__ __device__ constexpr int zg_min_blocks() { return zg_threads<BM, BN>() <= 256 ? 2 : 1; }
+__host__ __device__ constexpr int zg_min_blocks() { return zg_threads<BM, BN>() <= 64 ? 6 : (zg_threads<BM, BN>() <= 256 ? 2 : 1); }
+
+// Row pitches of the staged tiles (elements).  A 16-byte fragment load is served eight lanes at a time, and
+// lanes (fk, fr) of such a group read row kk + fk, column c + fr: with a pitch of 2 mod 8 they land on distinct
+// bank quadruples (one more than the tile, as before, made half of all shared-memory wavefronts conflicts).
+// An 8-byte load is served sixteen lanes at a time: 4 mod 16.
+template <bool AREAL>
+__host__ __device__ constexpr int zg_pitch_a(int bm) { return AREAL ? bm + 4 : bm + 2; }
+__host__ __device__ constexpr int zg_pitch_b(int bn) { return bn + 2; }
 
 template <bool AREAL>
 struct ATile {
     using T = typename std::conditional<AREAL, double, zc>::type;
 };
-
-__device__ __forceinline__ zc load_z(const View &v, long long off) {
-    if (v.real) return zc{reinterpret_cast<const double *>(v.p)[off], 0.0};
-    zc z = reinterpret_cast<const zc *>(v.p)[off];
-    if (v.conj) z.y = -z.y;
-    return z;
-}
-
-__device__ __forceinline__ double load_d(const View &v, long long off) {
-    return reinterpret_cast<const double *>(v.p)[off];
-}
 
 // D (8 x 8) += A (8 x 4, row-major) B (4 x 8, column-major), FP64.  Lane l holds A[l/4][l%4],
 // B[l%4][l/4] and D[l/4][2 (l%4) + {0, 1}].
@@ -67,7 +67,7 @@ __host__ __device__ constexpr int zg_stages() { return (BM == BN || BN == 112) ?
 template <bool AREAL, int BM, int BN>
 constexpr size_t zg_smem_bytes() {
     return (size_t)zg_stages<BM, BN>() * BK *
-           ((BM + 1) * (AREAL ? sizeof(double) : sizeof(zc)) + (BN + 1) * sizeof(zc));
+           (zg_pitch_a<AREAL>(BM) * (AREAL ? sizeof(double) : sizeof(zc)) + zg_pitch_b(BN) * sizeof(zc));
 }
 
 // BM x BN output tile, 256 threads = 8 warps of 32 x 16 (warp w: rows 32 (w / (BN/16)), columns
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     static_assert(BM % 32 == 0 && BN % 16 == 0, "tile/warp mismatch");
     // elements loaded per thread and k-tile (the last round partial when NT does not divide the tile)
     constexpr int LA = (BM * BK + NT - 1) / NT, LB = (BN * BK + NT - 1) / NT;
-    constexpr int PA = BM + 1, PB = BN + 1;                    // row pitches (elements)
+    constexpr int PA = zg_pitch_a<AREAL>(BM), PB = zg_pitch_b(BN);
     constexpr int ZG_STAGES = zg_stages<BM, BN>();
     extern __shared__ __align__(16) unsigned char zg_smem[];
     TA *As = reinterpret_cast<TA *>(zg_smem);                                      // [stage][kk][i]
@@ -108,46 +108,75 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     }
     const bool a_mfast = (A.rs == 1);  // element order of the A tile loads
     const bool b_nfast = (B.cs == 1);
-    const double sa = (!AREAL && A.conj) ? -1.0 : 1.0;  // imaginary-part signs (conjugated views)
-    const double sb = B.conj ? -1.0 : 1.0;
-    const uint32_t as_base = (uint32_t)__cvta_generic_to_shared(As);
-    const uint32_t bs_base = (uint32_t)__cvta_generic_to_shared(Bs);
     const int nkt = (k + BK - 1) / BK;
+    // Each thread's r-th element of a tile is dA rows (or k's) and a fixed pointer and shared-memory step after
+    // its first; the pointers advance by one k-tile per load_stage call (addresses from scratch for every
+    // element were three of five instructions of the k loop).
+    constexpr int RA = NT / BM, KA = NT / BK, RB = NT / BN;
+    static_assert(NT % BM == 0 && NT % BN == 0 && NT % BK == 0, "tile loads");
+    const int ai = a_mfast ? tid % BM : tid / BK, ak = a_mfast ? tid / BM : tid % BK;
+    const int bj = b_nfast ? tid % BN : tid / BK, bk = b_nfast ? tid / BN : tid % BK;
+    const int bsz = B.real ? (int)sizeof(double) : (int)sizeof(zc);
+    const unsigned char *pa = reinterpret_cast<const unsigned char *>(A.p) +
+                              (oa + (long long)(row0 + ai) * A.rs + (long long)ak * A.cs) * (long long)sizeof(TA);
+    const unsigned char *pb = reinterpret_cast<const unsigned char *>(B.p) +
+                              (ob + (long long)bk * B.rs + (long long)(col0 + bj) * B.cs) * bsz;
+    const long long astep = (long long)(a_mfast ? RA * A.cs : KA * A.rs) * (long long)sizeof(TA),
+                    bstep = (long long)(b_nfast ? RB * B.rs : KA * B.cs) * bsz;
+    const uint32_t sa0 = (uint32_t)__cvta_generic_to_shared(As) + (uint32_t)((ak * PA + ai) * sizeof(TA)),
+                   sar = (uint32_t)((a_mfast ? RA * PA : KA) * sizeof(TA));
+    const uint32_t sb0 = (uint32_t)__cvta_generic_to_shared(Bs) + (uint32_t)((bk * PB + bj) * sizeof(zc)),
+                   sbr = (uint32_t)((b_nfast ? RB * PB : KA) * sizeof(zc));
+    // bit r: the r-th element's row (column) is inside the matrix
+    unsigned amask = 0, bmask = 0;
+#pragma unroll
+    for (int r = 0; r < LA; ++r)
+        if (row0 + ai + (a_mfast ? 0 : KA * r) < m && ((BM * BK) % NT == 0 || tid + NT * r < BM * BK)) amask |= 1u << r;
+#pragma unroll
+    for (int r = 0; r < LB; ++r)
+        if (col0 + bj + (b_nfast ? 0 : KA * r) < n && ((BN * BK) % NT == 0 || tid + NT * r < BN * BK)) bmask |= 1u << r;
 
-    auto load_stage = [&](int stage, int kt) {
-        const int k0 = kt * BK;
+    auto load_stage = [&](int stage, int kt) {  // called for kt = 0, 1, 2, ... in turn
+        unsigned am = amask, bm = bmask;
+        if ((kt + 1) * BK > k) {  // the last k-tile
+            const int ka = k - kt * BK - ak, kb = k - kt * BK - bk;
+#pragma unroll
+            for (int r = 0; r < LA; ++r)
+                if ((a_mfast ? RA * r : 0) >= ka) am &= ~(1u << r);
+#pragma unroll
+            for (int r = 0; r < LB; ++r)
+                if ((b_nfast ? RB * r : 0) >= kb) bm &= ~(1u << r);
+        }
 #pragma unroll
         for (int r = 0; r < LA; ++r) {
-            const int e = tid + NT * r;
-            if ((BM * BK) % NT != 0 && e >= BM * BK) break;
-            int i, kk;
-            if (a_mfast) { i = e % BM; kk = e / BM; }
-            else { kk = e % BK; i = e / BK; }
-            const int gi = row0 + i, gk = k0 + kk;
-            const bool ok = gi < m && gk < k;
-            const long long off = ok ? oa + (long long)gi * A.rs + (long long)gk * A.cs : 0;
-            cp_async(as_base + (uint32_t)(((stage * BK + kk) * PA + i) * sizeof(TA)),
-                     reinterpret_cast<const unsigned char *>(A.p) + off * (long long)sizeof(TA),
-                     ok ? (int)sizeof(TA) : 0, (int)sizeof(TA));
+            if ((BM * BK) % NT != 0 && r == LA - 1 && tid + NT * r >= BM * BK) break;
+            const bool ok = (am >> r) & 1u;
+            cp_async(sa0 + (uint32_t)(stage * BK * PA * (int)sizeof(TA)) + r * sar,
+                     ok ? pa + r * astep : reinterpret_cast<const unsigned char *>(A.p), ok ? (int)sizeof(TA) : 0,
+                     (int)sizeof(TA));
         }
 #pragma unroll
         for (int r = 0; r < LB; ++r) {
-            const int e = tid + NT * r;
-            if ((BN * BK) % NT != 0 && e >= BN * BK) break;
-            int j, kk;
-            if (b_nfast) { j = e % BN; kk = e / BN; }
-            else { kk = e % BK; j = e / BK; }
-            const int gj = col0 + j, gk = k0 + kk;
-            const bool ok = gj < n && gk < k;
-            const long long off = ok ? ob + (long long)gk * B.rs + (long long)gj * B.cs : 0;
+            if ((BN * BK) % NT != 0 && r == LB - 1 && tid + NT * r >= BN * BK) break;
+            const bool ok = (bm >> r) & 1u;
+            const unsigned char *src = ok ? pb + r * bstep : reinterpret_cast<const unsigned char *>(B.p);
+            const uint32_t dst = sb0 + (uint32_t)(stage * BK * PB * (int)sizeof(zc)) + r * sbr;
             if (B.real) {
-                Bs[(stage * BK + kk) * PB + j] = zc{ok ? reinterpret_cast<const double *>(B.p)[off] : 0.0, 0.0};
+                const double x = ok ? *reinterpret_cast<const double *>(src) : 0.0;
+                asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(dst), "d"(x), "d"(0.0) : "memory");
             } else {
-                cp_async(bs_base + (uint32_t)(((stage * BK + kk) * PB + j) * sizeof(zc)),
-                         reinterpret_cast<const zc *>(B.p) + off, ok ? 16 : 0, 16);
+                cp_async(dst, src, ok ? 16 : 0, 16);
             }
         }
+        pa += (long long)BK * A.cs * (long long)sizeof(TA);
+        pb += (long long)BK * B.rs * bsz;
     };
+    // Signs of the imaginary parts (conjugated views): with sa, sb = +-1, cr = sum ax bx - sa sb ay by, and ci is
+    // accumulated as sb ci = sum ax by + sa sb ay bx, so that only A's fragments change sign.
+    const int neg = ((!AREAL && A.conj) != (B.conj != 0)) ? (int)0x80000000u : 0;
+    const auto flip = [](double x, int mask) { return __hiloint2double(__double2hiint(x) ^ mask, __double2loint(x)); };
+    // 8 x 8 blocks of this warp inside the matrix: the others (padding) are not multiplied
+    const int ni = min(4, (m - row0 - wr + 7) / 8), nj = min(2, (n - col0 - wc + 7) / 8);
 
     double cr[4][2][2], ci[4][2][2];  // 8 x 8 blocks (bi, bj): real and imaginary accumulators
 #pragma unroll
@@ -166,31 +195,38 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
         const int stage = kt % ZG_STAGES;
         const TA *At = As + (size_t)stage * BK * PA;
         const zc *Bt = Bs + (size_t)stage * BK * PB;
-#pragma unroll
-        for (int kk = 0; kk < BK; kk += 4) {
+        // one k-step of four; FULL: every block of the warp is inside the matrix
+        const auto step = [&](int kk, auto full) {
+            constexpr bool FULL = decltype(full)::value;
             zc b[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                b[j] = Bt[(kk + fk) * PB + wc + 8 * j + fr];
-                b[j].y *= sb;
-            }
+            for (int j = 0; j < 2; ++j) b[j] = Bt[(kk + fk) * PB + wc + 8 * j + fr];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                TA a = At[(kk + fk) * PA + wr + 8 * i + fr];
+                if (!FULL && i >= ni) break;
+                const TA a = At[(kk + fk) * PA + wr + 8 * i + fr];
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
+                    if (!FULL && j == 1 && nj < 2) break;
                     if constexpr (AREAL) {
                         dmma884(cr[i][j], a, b[j].x);
                         dmma884(ci[i][j], a, b[j].y);
                     } else {
-                        const double ay = a.y * sa;
                         dmma884(cr[i][j], a.x, b[j].x);
-                        dmma884(cr[i][j], -ay, b[j].y);
                         dmma884(ci[i][j], a.x, b[j].y);
-                        dmma884(ci[i][j], ay, b[j].x);
+                        dmma884(cr[i][j], flip(a.y, neg ^ (int)0x80000000u), b[j].y);
+                        dmma884(ci[i][j], flip(a.y, neg), b[j].x);
                     }
                 }
             }
+        };
+        const int krem = k - kt * BK;
+        if (ni == 4 && nj == 2 && krem >= BK) {
+#pragma unroll
+            for (int kk = 0; kk < BK; kk += 4) step(kk, std::true_type{});
+        } else if (nj > 0) {  // (warps, blocks and k-steps of padding alone are skipped)
+#pragma unroll 1
+            for (int kk = 0; kk < min(BK, krem); kk += 4) step(kk, std::false_type{});
         }
         const int kn = kt + ZG_STAGES - 1;  // refill the stage computed in the previous iteration
         if (kn < nkt) load_stage(kn % ZG_STAGES, kn);
@@ -203,21 +239,32 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
         const int gi = row0 + wr + 8 * i + fr;
         if (gi >= m) continue;
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < 2; ++j) {
+            const int gj = col0 + wc + 8 * j + 2 * fk;
+            if (gj >= n) continue;
+            zc v[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[h] = alpha * zc{cr[i][j][h], B.conj ? -ci[i][j][h] : ci[i][j][h]};
+            const long long off = oc + (long long)gi * C.rs + (long long)gj * C.cs;
+            // consecutive columns side by side: one 32-byte store (a whole sector) instead of two halves
+            if (!C.real && !use_beta && C.cs == 1 && gj + 1 < n && (reinterpret_cast<uintptr_t>(C.p + off) & 31) == 0) {
+                asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(C.p + off), "d"(v[0].x), "d"(v[0].y),
+                             "d"(v[1].x), "d"(v[1].y)
+                             : "memory");
+                continue;
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int gj = col0 + wc + 8 * j + 2 * fk + h;
-                if (gj >= n) continue;
-                long long off = oc + (long long)gi * C.rs + (long long)gj * C.cs;
-                zc v = alpha * zc{cr[i][j][h], ci[i][j][h]};
+                if (gj + h >= n) continue;
+                const long long o = off + h * C.cs;
                 if (C.real) {
                     double *cp = reinterpret_cast<double *>(C.p);
-                    cp[off] = use_beta ? v.x + beta.x * cp[off] : v.x;
+                    cp[o] = use_beta ? v[h].x + beta.x * cp[o] : v[h].x;
                 } else {
-                    if (use_beta) v = v + beta * C.p[off];
-                    C.p[off] = v;
+                    C.p[o] = use_beta ? v[h] + beta * C.p[o] : v[h];
                 }
             }
+        }
     }
 }
 
@@ -252,13 +299,14 @@ int launch_tile(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, 
     return PHF_OK;
 }
 
-// Tile shape 0 = 64 x 64, 1 = 128 x 32, 2 = 32 x 128, 3 = 32 x 112, 4 = 64 x 112.
+// Tile shape 0 = 64 x 64, 1 = 128 x 32, 2 = 32 x 128, 3 = 32 x 112, 4 = 64 x 112, 5 = 32 x 32.
 int launch_choice(int tile, int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, const View &B, zc beta,
                   const OutView &C, const long long *offs, cudaStream_t st) {
     if (tile == 1) return launch_tile<128, 32>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     if (tile == 2) return launch_tile<32, 128>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     if (tile == 3) return launch_tile<32, 112>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     if (tile == 4) return launch_tile<64, 112>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
+    if (tile == 5) return launch_tile<32, 32>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     return launch_tile<64, 64>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
 }
 
@@ -278,11 +326,22 @@ int zgemm_strided(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A
     const TuneKey key{0, (long long)m, (long long)n, (long long)k, (long long)nb0 * 65536 + nb1,
                       (long long)(A.real * 4 + B.real * 2 + C.real) * 2 + (offs != nullptr)};
     if (t_tune_record)
-        t_tune_record->push_back({key, {0, 1, 2, 3, 4}, [=](int tile, cudaStream_t s) {
+        t_tune_record->push_back({key, {0, 1, 2, 3, 4, 5}, [=](int tile, cudaStream_t s) {
                                       return launch_choice(tile, m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, s);
                                   }});
     int tile = tuned_choice(key);
-    if (tile < 0) tile = (n <= 32 && m >= 96) ? 1 : ((m <= 32 && n >= 96) ? 2 : ((n > 96 && n <= 112) ? 3 : 0));
+    if (tile < 0) {
+        tile = (n <= 32 && m >= 96) ? 1 : ((m <= 32 && n >= 96) ? 2 : ((n > 96 && n <= 112) ? 3 : 0));
+        // 32 x 32 tiles where the larger tile leaves multiprocessors idle or is mostly padding: the FP64 units of
+        // one multiprocessor run at 64 multiply-adds a cycle whatever the tile, so the time goes with the
+        // output elements per multiprocessor.  A quarter is allowed for the smaller tile's extra loads.
+        constexpr int bm[4] = {64, 128, 32, 32}, bn[4] = {64, 32, 128, 112};
+        const auto load = [&](int r, int c) {
+            const long long ctas = (long long)nb0 * nb1 * ((m + r - 1) / r) * ((n + c - 1) / c);
+            return (double)((ctas + 147) / 148) * r * c;
+        };
+        if (1.25 * load(32, 32) < load(bm[tile], bn[tile]) && (m + 31) / 32 <= 65535) tile = 5;
+    }
     return launch_choice(tile, m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
 }
 
