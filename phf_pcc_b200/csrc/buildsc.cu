@@ -13,6 +13,13 @@
 // are strided batched FP64 GEMMs on the tensor cores (zgemm_strided), the M^4 index permutations,
 // outer products and two-index contractions are the elementwise kernels below.  Tensors follow the
 // Fortran arrays: X(a, b, c, d) at a + M b + M^2 c + M^3 d, X(a, b) at a + M b.
+//
+// Everything between a point's four-index products and the sum over points is linear, so the weighted sums
+// over the points are taken first and the index permutations of t2 once at the end (one kernel over M^4
+// elements): sum_w s_w tau12_w and sum_w s_w tau20_w are single GEMMs with the contraction over (point, e), and
+// the outer products sum_w s_w Y_w (x) Z_w are GEMMs with the points as the contraction index.  Per point only
+// the four-index products, tau19 and two contractions remain.  (Assembling t2 point by point took 28 of the
+// 44 ms of 112 points at M = 32, in 172 passes over M^4 elements; now the whole sequence takes 15.6 ms.)
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -55,33 +62,54 @@ __global__ void axpy4_kernel(int n0, int n1, int n2, int n3, int b, zc *out, S4 
     }
 }
 
-// out(a,b,c,d)_w = [init ? 0 : out] + sign alpha_w X(.)_w Z(.)_w   (X and Z each use two of the indices)
-__global__ void outer4_kernel(int M, int b, zc *out, const zc *X, S4 xs, const zc *Z, S4 zs, const zc *alpha,
-                              double sign, int init) {
-    const long long M4 = (long long)M * M * M * M, tot = M4 * b;
-    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < tot; e += (long long)gridDim.x * NT) {
-        const long long w = e / M4, r = e - w * M4;
-        const int a = (int)(r % M), bb = (int)((r / M) % M), c = (int)((r / ((long long)M * M)) % M),
-                  d = (int)(r / ((long long)M * M * M));
-        const zc x = X[a * xs.s[0] + bb * xs.s[1] + c * xs.s[2] + d * xs.s[3] + w * xs.w];
-        const zc z = Z[a * zs.s[0] + bb * zs.s[1] + c * zs.s[2] + d * zs.s[3] + w * zs.w];
-        zc v = sign * (x * z);
-        if (alpha) v = alpha[w] * v;
-        out[e] = init ? v : out[e] + v;
+// out(a, b, c, d)_w = in(a, b, d, c)_w - in(a, b, c, d)_w
+__global__ void swap_last_kernel(int M, long long n, const zc *__restrict__ in, zc *__restrict__ out) {
+    const long long M2 = (long long)M * M;
+    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < n; e += (long long)gridDim.x * NT) {
+        const long long ab = e % M2, r = e / M2;  // r = c + M d + M^2 w
+        const int c = (int)(r % M), d = (int)((r / M) % M);
+        out[e] = in[ab + M2 * (r + (long long)(d - c) + (long long)M * (c - d))] - in[e];
     }
 }
 
-// out(a, b)_w = [init ? 0 : out] + sign sum_{c,d} Y(c, d)_w T(a, b, c, d)_w  (T read with strides ts)
-__global__ void contract2_kernel(int M, zc *out, const zc *Y, const zc *T, S4 ts, double sign, int init) {
+// t2 from the weighted sums over the points: s12 = sum s tau12, s20 = sum s tau20, s10 = sum s tau10 and, at
+// (x + M y) + M^2 (p + M q), g = sum s Y(x, y) Z(p, q) for Z = tau8 Y - tau18 + tau17^T (g1), tau27, tau15, tau21:
+//   tau16 = s12 - g15[(a, c), (d, b)],   tau22 = -s20 + g21[(a, b), (c, d)]
+__global__ void assemble_t2_kernel(int M, const zc *__restrict__ s12, const zc *__restrict__ s20,
+                                   const zc *__restrict__ s10, const zc *__restrict__ g1, const zc *__restrict__ g27,
+                                   const zc *__restrict__ g15, const zc *__restrict__ g21, zc *__restrict__ t2) {
+    const long long M1 = M, M2 = M1 * M, M3 = M2 * M, M4 = M2 * M2;
+    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < M4; e += (long long)gridDim.x * NT) {
+        const long long a = e % M, b = (e / M) % M, c = (e / M2) % M, d = e / M3;
+        const auto at = [&](const zc *X, long long i, long long j, long long k, long long l) {
+            return X[i + M1 * j + M2 * k + M3 * l];
+        };
+        const auto t16 = [&](long long i, long long j, long long k, long long l) {
+            return at(s12, i, j, k, l) - at(g15, i, k, l, j);
+        };
+        const auto t22 = [&](long long i, long long j, long long k, long long l) {
+            return at(g21, i, j, k, l) - at(s20, i, j, k, l);
+        };
+        zc v = at(g1, a, c, b, d) - at(g1, b, c, a, d);
+        v = v + (at(g27, b, d, c, a) - at(g27, a, d, c, b));
+        v = v + (t16(a, b, c, d) - t16(a, b, d, c) - t16(b, a, c, d) + t16(b, a, d, c));
+        v = v + (t22(a, c, d, b) - t22(a, d, c, b) - t22(b, c, d, a) + t22(b, d, c, a));
+        v = v + (at(s10, c, d, a, b) - at(s10, c, d, b, a) - at(s10, d, c, a, b) + at(s10, d, c, b, a));
+        t2[e] = v;
+    }
+}
+
+// out(a, b)_w = sum_{c,d} Y(c, d)_w (T(.)_w - T(.)_w), T read with the strides ts and us over (a, b, c, d)
+__global__ void contract2_kernel(int M, zc *out, const zc *Y, const zc *T, S4 ts, S4 us) {
     __shared__ zc sh[NT];
     const int a = blockIdx.x % M, bb = blockIdx.x / M;
     const long long w = blockIdx.y;
     const zc *y = Y + w * (long long)M * M;
-    const zc *t = T + w * ts.w + a * ts.s[0] + bb * ts.s[1];
+    const zc *t = T + w * ts.w + a * ts.s[0] + bb * ts.s[1], *u = T + w * us.w + a * us.s[0] + bb * us.s[1];
     zc acc = mkz(0, 0);
     for (int e = threadIdx.x; e < M * M; e += NT) {
         const int c = e % M, d = e / M;
-        acc = acc + y[c + (long long)M * d] * t[c * ts.s[2] + d * ts.s[3]];
+        acc = acc + y[c + (long long)M * d] * (t[c * ts.s[2] + d * ts.s[3]] - u[c * us.s[2] + d * us.s[3]]);
     }
     sh[threadIdx.x] = acc;
     __syncthreads();
@@ -89,11 +117,7 @@ __global__ void contract2_kernel(int M, zc *out, const zc *Y, const zc *T, S4 ts
         if (threadIdx.x < s) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + s];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        zc *o = out + w * (long long)M * M + a + (long long)M * bb;
-        const zc v = sign * sh[0];
-        *o = init ? v : *o + v;
-    }
+    if (threadIdx.x == 0) out[w * (long long)M * M + a + (long long)M * bb] = sh[0];
 }
 
 // out_w = [init ? 0 : out_w] + sign sum_{a,b} X(a, b)_w Z(.)_w  (X plain M x M, Z with strides zs over (a, b))
@@ -182,20 +206,6 @@ struct Ctx {
         for (int pos = 0; pos < 4; ++pos) s.s[p[pos] - 'a'] += str[pos];
         return s;
     }
-    // a two-index operand X(i, j) over the output's loop indices: i, j name which of a..d
-    S4 two(char i, char j) const {
-        S4 s{{0, 0, 0, 0}, M2()};
-        s.s[i - 'a'] += 1;
-        s.s[j - 'a'] += M;
-        return s;
-    }
-    int axpy4(zc *out, const zc *in, const char *p, double sign, int init, const zc *alpha = nullptr) const {
-        S4 os{{1, M, M2(), M3()}, M4()};
-        axpy4_kernel<<<blocks_for(M4() * b), NT, 0, st>>>(M, M, M, M, b, out, os, in, perm(p), alpha, sign, init);
-        ++g_launches;
-        PHF_CHECK_LAUNCH();
-        return PHF_OK;
-    }
     // two-index axpy: out(a, b) (+)= sign alpha in(a, b) or in(b, a) (transposed)
     int axpy2(zc *out, const zc *in, bool transposed, double sign, int init, const zc *alpha = nullptr) const {
         S4 os{{1, M, 0, 0}, M2()};
@@ -205,19 +215,21 @@ struct Ctx {
         PHF_CHECK_LAUNCH();
         return PHF_OK;
     }
-    int outer4(zc *out, const zc *X, S4 xs, const zc *Z, S4 zs, double sign, int init,
-               const zc *alpha = nullptr) const {
-        outer4_kernel<<<blocks_for(M4() * b), NT, 0, st>>>(M, b, out, X, xs, Z, zs, alpha, sign, init);
+    // out(a, b) = sum_{c,d} Y(c, d) (T(q) - T(r)) with q, r the index orders of T over (a, b, c, d)
+    int contract2(zc *out, const zc *Y, const zc *T, const char *q, const char *r) const {
+        contract2_kernel<<<dim3((unsigned)(M * M), (unsigned)b), NT, 0, st>>>(M, out, Y, T, perm(q), perm(r));
         ++g_launches;
         PHF_CHECK_LAUNCH();
         return PHF_OK;
     }
-    // out(a, b) (+)= sign sum_{c,d} Y(c, d) T(q) with q the index order of T over (a, b, c, d)
-    int contract2(zc *out, const zc *Y, const zc *T, const char *q, double sign, int init) const {
-        contract2_kernel<<<dim3((unsigned)(M * M), (unsigned)b), NT, 0, st>>>(M, out, Y, T, perm(q), sign, init);
-        ++g_launches;
-        PHF_CHECK_LAUNCH();
-        return PHF_OK;
+    // acc(a, b, c, d) += sum over the points and e of Ys(a, e) X(b, c, d, e): one GEMM, contraction (point, e)
+    int gemm4_sum(zc *acc, const zc *Ys, const zc *X) const {
+        return zgemm_strided((int)M3(), M, M * b, 1, 1, ONE, V(X, 1, M3()), V(Ys, M, 1), ONE, O(acc, M, 1), nullptr, st);
+    }
+    // acc[(x, y), (p, q)] += sum over the points of Ys(x, y) Z(p, q)
+    int outer_sum(zc *acc, const zc *Ys, const zc *Z) const {
+        return zgemm_strided((int)M2(), (int)M2(), b, 1, 1, ONE, V(Ys, 1, M2()), V(Z, M2(), 1), ONE, O(acc, 1, M2()),
+                             nullptr, st);
     }
     // out_w (+)= sign sum_{a,b} X(a, b) Z(a, b) or Z(b, a)
     int trace2(zc *out, const zc *X, const zc *Z, bool transposed, double sign, int init) const {
@@ -266,10 +278,10 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
                                std::conj(cd(fpg[p].re, fpg[p].im)) * cd(fpg[q].re, fpg[q].im);
                 wt[((size_t)il * ny + iy) * npg + ig] = weightsp[(size_t)il + (size_t)nl * iy] * wpg * fsc * fs;
             }
-    // chunk from the workspace budget: eight M^4 and about twenty M^2 tensors per point
-    const size_t per = (8 * (size_t)M4 + 24 * (size_t)M2 + (size_t)N * N + 16) * sizeof(zc);
+    // chunk from the workspace budget: three M^4 and about twenty M^2 tensors per point
+    const size_t per = (3 * (size_t)M4 + 24 * (size_t)M2 + (size_t)N * N + 16) * sizeof(zc);
     const size_t budget = workspace ? workspace : ((size_t)4 << 30);
-    const int b = (int)std::max<size_t>(1, std::min<size_t>(budget / per, (size_t)nw));
+    const int b = (int)std::max<size_t>(1, std::min<size_t>({budget / per, (size_t)nw, (size_t)65535}));
 
     Arena ar;
     zc *R1 = nullptr, *R2 = nullptr, *Rpg = nullptr, *c1 = nullptr, *c2 = nullptr, *wtd = nullptr;
@@ -315,7 +327,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     zc *T = nullptr, *R = nullptr, *Sinv = nullptr, *det = nullptr, *logdet = nullptr, *Y = nullptr, *c1t = nullptr,
        *t2d = nullptr, *sc = nullptr, *sclr = nullptr, *acc0 = nullptr, *acc1 = nullptr, *acc2 = nullptr,
        *ovlp = nullptr;
-    zc *B4[7] = {};
+    zc *B4[3] = {}, *S4sum[7] = {};  // weighted sums over the points: s12, s20, s10, g1, g27, g15, g21
     zc *B2[18] = {};
     int *flag = nullptr;
     PHF_TRY(ar.alloc(&T, (size_t)b * M2));
@@ -329,6 +341,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     PHF_TRY(ar.alloc(&sc, (size_t)b));
     PHF_TRY(ar.alloc(&sclr, 4 * (size_t)b));
     for (auto &p : B4) PHF_TRY(ar.alloc(&p, (size_t)b * M4));
+    for (auto &p : S4sum) PHF_TRY(ar.alloc(&p, (size_t)M4));
     for (auto &p : B2) PHF_TRY(ar.alloc(&p, (size_t)b * M2));
     PHF_TRY(ar.alloc(&acc0, 1));
     PHF_TRY(ar.alloc(&acc1, (size_t)M2));
@@ -338,15 +351,14 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     cudaStream_t st = 0;
     PHF_CUDA(cudaMemsetAsync(acc0, 0, sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(acc1, 0, M2 * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(acc2, 0, M4 * sizeof(zc), st));
+    for (auto &p : S4sum) PHF_CUDA(cudaMemsetAsync(p, 0, M4 * sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(ovlp, 0, sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
     // four-index buffers (reused as the sequence allows) and two-index intermediates
-    zc *c2t = B4[0], *tau11 = B4[0], *tmp = B4[1], *tau9 = B4[1], *tau19 = B4[1], *tau0 = B4[2], *tau10 = B4[3],
-       *tau16 = B4[4], *tau22 = B4[5], *a2 = B4[6];
+    zc *c2t = B4[0], *tau11 = B4[0], *tmp = B4[1], *tau9 = B4[1], *tau19 = B4[1], *tau10 = B4[2];
     zc *tau1 = B2[0], *tau2 = B2[1], *tau5 = B2[2], *tau6 = B2[3], *tau7 = B2[4], *tau13 = B2[5], *tau14 = B2[6],
        *tau15 = B2[7], *tau17 = B2[8], *tau18 = B2[9], *tau21 = B2[10], *tau24 = B2[11], *tau25 = B2[12],
-       *tau26 = B2[13], *tau27 = B2[14], *a1 = B2[15];
+       *tau26 = B2[13], *tau27 = B2[14], *a1 = B2[15], *Ys = B2[16], *Z1 = B2[17];
     zc *tau3 = sclr, *tau8 = sclr + b, *tau23 = sclr + 2 * (size_t)b, *a0 = sclr + 3 * (size_t)b;
     const zc c0{c0h.re, c0h.im};
 
@@ -379,23 +391,23 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
                               nullptr, st));  // (i,j,k,l) = sum_x conj U(x,i) (x,j,k,l)
 
         // ---- BuildSC_Vec (PHF_fort/BuildSC_dr.f90), Y = the transition density of each point
-        PHF_TRY(x.axpy4(tau0, c2t, "abcd", 1.0, 1));
-        PHF_TRY(x.axpy4(tau0, c2t, "bacd", -1.0, 0));
-        PHF_TRY(x.contract2(tau1, Y, tau0, "dabc", 1.0, 1));                 // tau1 = Y(c,d) tau0(d,a,b,c)
+        // weights s_w = det S_w weightsp wpg (...) of the points, and s_w Y_w
+        weights_kernel<<<(bc + NT - 1) / NT, NT, 0, st>>>(bc, w0, det, wtd, sc, ovlp);
+        ++g_launches;
+        PHF_CHECK_LAUNCH();
+        PHF_TRY(x.axpy2(Ys, Y, false, 1.0, 1, sc));
+        // tau0(a,b,c,d) = c2(a,b,c,d) - c2(b,a,c,d), read in place
+        PHF_TRY(x.contract2(tau1, Y, c2t, "dabc", "adbc"));                  // tau1 = Y(c,d) tau0(d,a,b,c)
         PHF_TRY(x.axpy2(tau2, tau1, false, -1.0, 1));
         PHF_TRY(x.axpy2(tau6, tau1, false, -1.0, 1));
         PHF_TRY(x.trace2(tau8, Y, tau1, true, -1.0, 1));                      // tau8 = -Y(a,b) tau1(b,a)
-        PHF_TRY(x.outer4(a2, Y, x.two('a', 'c'), Y, x.two('b', 'd'), 1.0, 1, tau8));
-        PHF_TRY(x.outer4(a2, Y, x.two('a', 'd'), Y, x.two('b', 'c'), -1.0, 0, tau8));
         PHF_TRY(x.axpy2(tau13, tau1, false, -1.0, 1));
-        PHF_TRY(x.contract2(tau5, Y, tau0, "adcb", 1.0, 1));                 // tau5 = Y(c,d) tau0(a,d,c,b)
+        PHF_TRY(x.contract2(tau5, Y, c2t, "adcb", "dacb"));                  // tau5 = Y(c,d) tau0(a,d,c,b)
         PHF_TRY(x.axpy2(tau6, tau5, false, -1.0, 0));
         PHF_TRY(x.axpy2(tau13, tau5, false, -1.0, 0));
         PHF_TRY(x.gemm2(tau14, V(Y, 1, M, M2), V(tau13, 1, M, M2)));         // Y(a,c) tau13(c,b)
         PHF_TRY(x.gemm2(tau15, V(Y, M, 1, M2), V(tau14, M, 1, M2)));         // Y(c,a) tau14(b,c)
-        PHF_TRY(x.outer4(tau16, Y, x.two('a', 'c'), tau15, x.two('d', 'b'), -1.0, 1));
         PHF_TRY(x.gemm2(tau21, V(Y, M, 1, M2), V(tau13, M, 1, M2)));         // Y(c,a) tau13(b,c)
-        PHF_TRY(x.outer4(tau22, Y, x.two('a', 'b'), tau21, x.two('c', 'd'), 1.0, 1));
         PHF_TRY(x.axpy2(tau2, c1t, false, 1.0, 0));
         PHF_TRY(x.trace2(tau3, Y, tau2, true, 1.0, 1));                       // tau3 = Y(a,b) tau2(b,a)
         PHF_TRY(x.axpy2(a1, Y, false, 1.0, 1, tau3));                         // t1 = tau3 Y
@@ -409,28 +421,19 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         PHF_TRY(x.gemm4(tau9, Y, false, c2t));                                // Y(e,a) c2(b,c,d,e)
         PHF_TRY(x.gemm4(tau10, Y, false, tau9));                              // Y(e,a) tau9(b,c,d,e)
         PHF_TRY(x.gemm4(tau11, Y, true, tau10));                              // Y(a,e) tau10(b,c,d,e)
-        PHF_TRY(x.gemm4(tau16, Y, true, tau11, ONE, ONE));                    // + tau12 = Y(a,e) tau11(b,c,d,e)
-        PHF_TRY(x.axpy4(a2, tau16, "abcd", 1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau16, "abdc", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau16, "bacd", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau16, "badc", 1.0, 0));
-        PHF_TRY(x.axpy4(tau19, tau10, "abcd", -1.0, 1));
-        PHF_TRY(x.axpy4(tau19, tau10, "abdc", 1.0, 0));
-        PHF_TRY(x.gemm4(tau22, Y, true, tau19, MONE, ONE));                   // - tau20 = Y(a,e) tau19(b,c,d,e)
-        PHF_TRY(x.axpy4(a2, tau22, "acdb", 1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau22, "adcb", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau22, "bcda", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau22, "bdca", 1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau10, "cdab", 1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau10, "cdba", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau10, "dcab", -1.0, 0));
-        PHF_TRY(x.axpy4(a2, tau10, "dcba", 1.0, 0));
+        PHF_TRY(x.gemm4_sum(S4sum[0], Ys, tau11));                            // s12: tau12 = Y(a,e) tau11(b,c,d,e)
+        swap_last_kernel<<<blocks_for(M4 * bc), NT, 0, st>>>(M, M4 * bc, tau10, tau19);  // tau10(abdc) - tau10(abcd)
+        ++g_launches;
+        PHF_CHECK_LAUNCH();
+        PHF_TRY(x.gemm4_sum(S4sum[1], Ys, tau19));                            // s20: tau20 = Y(a,e) tau19(b,c,d,e)
+        accumulate_kernel<<<blocks_for(M4), NT, 0, st>>>(M4, bc, tau10, sc, S4sum[2]);  // s10
+        ++g_launches;
+        PHF_CHECK_LAUNCH();
         PHF_TRY(x.gemm2(tau17, V(Y, M, 1, M2), V(c1t, M, 1, M2)));           // Y(c,a) c1(b,c)
         PHF_TRY(x.gemm2(tau18, V(Y, 1, M, M2), V(tau17, M, 1, M2)));         // Y(a,c) tau17(b,c)
-        PHF_TRY(x.outer4(a2, Y, x.two('a', 'c'), tau18, x.two('b', 'd'), -1.0, 0));
-        PHF_TRY(x.outer4(a2, Y, x.two('b', 'c'), tau18, x.two('a', 'd'), 1.0, 0));
-        PHF_TRY(x.outer4(a2, Y, x.two('a', 'c'), tau17, x.two('d', 'b'), 1.0, 0));
-        PHF_TRY(x.outer4(a2, Y, x.two('b', 'c'), tau17, x.two('d', 'a'), -1.0, 0));
+        PHF_TRY(x.axpy2(Z1, Y, false, 1.0, 1, tau8));                         // tau8 Y(b,d) - tau18(b,d) + tau17(d,b)
+        PHF_TRY(x.axpy2(Z1, tau18, false, -1.0, 0));
+        PHF_TRY(x.axpy2(Z1, tau17, true, 1.0, 0));
         PHF_TRY(x.trace2(tau23, Y, c1t, true, 1.0, 1));                       // tau23 = Y(b,a) c1(a,b)
         PHF_TRY(x.axpy2(tau27, Y, true, 1.0, 1, tau23));                      // tau27 = tau23 Y(b,a)
         PHF_TRY(x.gemm2(tau24, V(Y, 1, M, M2), V(c1t, 1, M, M2)));           // Y(a,c) c1(c,b)
@@ -450,19 +453,19 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
             ++g_launches;
             PHF_CHECK_LAUNCH();
         }
-        PHF_TRY(x.outer4(a2, Y, x.two('b', 'd'), tau27, x.two('c', 'a'), 1.0, 0));
-        PHF_TRY(x.outer4(a2, Y, x.two('a', 'd'), tau27, x.two('c', 'b'), -1.0, 0));
+        const zc *Zs[4] = {Z1, tau27, tau15, tau21};
+        for (int z = 0; z < 4; ++z) PHF_TRY(x.outer_sum(S4sum[3 + z], Ys, Zs[z]));
 
-        // ---- weights and accumulation over the chunk's points (fixed order)
-        weights_kernel<<<(bc + NT - 1) / NT, NT, 0, st>>>(bc, w0, det, wtd, sc, ovlp);
-        ++g_launches;
-        PHF_CHECK_LAUNCH();
+        // ---- accumulation of the smaller parts over the chunk's points (fixed order)
         accumulate_kernel<<<1, NT, 0, st>>>(1, bc, a0, sc, acc0);
         accumulate_kernel<<<blocks_for(M2), NT, 0, st>>>(M2, bc, a1, sc, acc1);
-        accumulate_kernel<<<blocks_for(M4), NT, 0, st>>>(M4, bc, a2, sc, acc2);
-        g_launches += 3;
+        g_launches += 2;
         PHF_CHECK_LAUNCH();
     }
+    assemble_t2_kernel<<<blocks_for(M4), NT, 0, st>>>(M, S4sum[0], S4sum[1], S4sum[2], S4sum[3], S4sum[4], S4sum[5],
+                                                      S4sum[6], acc2);
+    ++g_launches;
+    PHF_CHECK_LAUNCH();
     std::vector<cd> h0(1), h1(M2), h2(M4), ho(1);
     int hflag = 0;
     PHF_CUDA(cudaMemcpyAsync(h0.data(), acc0, sizeof(zc), cudaMemcpyDeviceToHost, st));
