@@ -75,10 +75,12 @@ __global__ void swap_last_kernel(int M, long long n, const zc *__restrict__ in, 
 // t2 from the weighted sums over the points: s12 = sum s tau12, s20 = sum s tau20, s10 = sum s tau10 and, at
 // (x + M y) + M^2 (p + M q), g = sum s Y(x, y) Z(p, q) for Z = tau8 Y - tau18 + tau17^T (g1), tau27, tau15, tau21:
 //   tau16 = s12 - g15[(a, c), (d, b)],   tau22 = -s20 + g21[(a, b), (c, d)]
-__global__ void assemble_t2_kernel(int M, const zc *__restrict__ s12, const zc *__restrict__ s20,
+// divided by the projected overlap.
+__global__ void assemble_t2_kernel(int M, const zc *__restrict__ ovlp, const zc *__restrict__ s12, const zc *__restrict__ s20,
                                    const zc *__restrict__ s10, const zc *__restrict__ g1, const zc *__restrict__ g27,
                                    const zc *__restrict__ g15, const zc *__restrict__ g21, zc *__restrict__ t2) {
     const long long M1 = M, M2 = M1 * M, M3 = M2 * M, M4 = M2 * M2;
+    const zc ov = *ovlp;
     for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < M4; e += (long long)gridDim.x * NT) {
         const long long a = e % M, b = (e / M) % M, c = (e / M2) % M, d = e / M3;
         const auto at = [&](const zc *X, long long i, long long j, long long k, long long l) {
@@ -95,7 +97,7 @@ __global__ void assemble_t2_kernel(int M, const zc *__restrict__ s12, const zc *
         v = v + (t16(a, b, c, d) - t16(a, b, d, c) - t16(b, a, c, d) + t16(b, a, d, c));
         v = v + (t22(a, c, d, b) - t22(a, d, c, b) - t22(b, c, d, a) + t22(b, d, c, a));
         v = v + (at(s10, c, d, a, b) - at(s10, c, d, b, a) - at(s10, d, c, a, b) + at(s10, d, c, b, a));
-        t2[e] = v;
+        t2[e] = divz(v, ov);
     }
 }
 
@@ -281,9 +283,11 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     // chunk from the workspace budget: three M^4 and about twenty M^2 tensors per point
     const size_t per = (3 * (size_t)M4 + 24 * (size_t)M2 + (size_t)N * N + 16) * sizeof(zc);
     const size_t budget = workspace ? workspace : ((size_t)4 << 30);
-    const int b = (int)std::max<size_t>(1, std::min<size_t>({budget / per, (size_t)nw, (size_t)65535}));
+    const int bmax = (int)std::max<size_t>(1, std::min<size_t>({budget / per, (size_t)nw, (size_t)65535}));
+    const int b = (nw + (nw + bmax - 1) / bmax - 1) / ((nw + bmax - 1) / bmax);  // equal chunks
 
     Arena ar;
+    ar.pooled = true;
     zc *R1 = nullptr, *R2 = nullptr, *Rpg = nullptr, *c1 = nullptr, *c2 = nullptr, *wtd = nullptr;
     long long *offs = nullptr;
     // rotations column-major per index: R(i, j) at i + M j
@@ -462,15 +466,14 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         g_launches += 2;
         PHF_CHECK_LAUNCH();
     }
-    assemble_t2_kernel<<<blocks_for(M4), NT, 0, st>>>(M, S4sum[0], S4sum[1], S4sum[2], S4sum[3], S4sum[4], S4sum[5],
+    assemble_t2_kernel<<<blocks_for(M4), NT, 0, st>>>(M, ovlp, S4sum[0], S4sum[1], S4sum[2], S4sum[3], S4sum[4], S4sum[5],
                                                       S4sum[6], acc2);
     ++g_launches;
     PHF_CHECK_LAUNCH();
-    std::vector<cd> h0(1), h1(M2), h2(M4), ho(1);
+    std::vector<cd> h0(1), h1(M2), ho(1);
     int hflag = 0;
     PHF_CUDA(cudaMemcpyAsync(h0.data(), acc0, sizeof(zc), cudaMemcpyDeviceToHost, st));
     PHF_CUDA(cudaMemcpyAsync(h1.data(), acc1, M2 * sizeof(zc), cudaMemcpyDeviceToHost, st));
-    PHF_CUDA(cudaMemcpyAsync(h2.data(), acc2, M4 * sizeof(zc), cudaMemcpyDeviceToHost, st));
     PHF_CUDA(cudaMemcpyAsync(ho.data(), ovlp, sizeof(zc), cudaMemcpyDeviceToHost, st));
     PHF_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     PHF_CUDA(cudaStreamSynchronize(st));
@@ -491,11 +494,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         t1h[i].re = v.real();
         t1h[i].im = v.imag();
     }
-    for (long long i = 0; i < M4; ++i) {
-        const cd v = h2[i] / ov;
-        t2h[i].re = v.real();
-        t2h[i].im = v.imag();
-    }
+    PHF_CUDA(cudaMemcpy(t2h, acc2, M4 * sizeof(zc), cudaMemcpyDeviceToHost));
     return PHF_OK;
 }
 

@@ -845,9 +845,11 @@ int pbarhbarolap_run(const PccArgs &g, phf_complex *olap0, phf_complex *olapex1,
                                 8 * M2 + 12 * vo + 4 * (long long)v * v + 4 * (long long)o * o + 32) *
                        sizeof(zc);
     const size_t budget = g.workspace ? g.workspace : ((size_t)16 << 30);
-    const int b = (int)std::max<size_t>(1, std::min<size_t>(budget / per, (size_t)nw));
+    const int bmax = (int)std::max<size_t>(1, std::min<size_t>(budget / per, (size_t)nw));
+    const int b = (nw + (nw + bmax - 1) / bmax - 1) / ((nw + bmax - 1) / bmax);  // equal chunks
 
     Arena ar;
+    ar.pooled = true;
     zc *H1 = nullptr, *H2 = nullptr, *T1 = nullptr, *T2 = nullptr, *R1 = nullptr, *R2 = nullptr, *Rpg = nullptr,
        *Rk2 = nullptr, *wtd = nullptr, *one = nullptr;
     long long *offs = nullptr;

@@ -107,7 +107,7 @@ int phf_buildhsg(const phf_complex *hone, const phf_complex *htwo, const phf_com
     d.htwo = htwo;
     d.precision = PHF_PREC_FP64;
     phf_plan *plan = nullptr;
-    int st = phf::plan_create(&d, &plan);
+    int st = phf::plan_create(&d, &plan, true);
     if (st != PHF_OK) return st;
     st = phf::plan_buildhsg(plan->impl, z, hmat, smat, gradmat, rdmmat);
     phf_plan_destroy(plan);
@@ -133,7 +133,7 @@ int phf_buildhsg_chol(const double *h, const double *bvec, int nchol, const phf_
     d.bvec = bvec;
     d.precision = precision;
     phf_plan *plan = nullptr;
-    int st = phf::plan_create(&d, &plan);
+    int st = phf::plan_create(&d, &plan, true);
     if (st != PHF_OK) return st;
     st = phf::plan_buildhsg(plan->impl, z, hmat, smat, gradmat, rdmmat);
     phf_plan_destroy(plan);
@@ -195,42 +195,28 @@ int phf_localg(const phf_complex *gradmat, const phf_complex *rdmmat, const phf_
                 }
     const long long MM = (long long)nso * nso, ns = (long long)nci * nci;
     const int nterm = (int)cg.size();
+    phf::Arena ar;
+    ar.pooled = true;
     phf::zc *dg = nullptr, *dr = nullptr, *dG = nullptr, *dcg = nullptr, *dcr = nullptr;
     long long *dslot = nullptr;
     int *dcj = nullptr;
-    int st = PHF_OK;
-    auto fail = [&](const char *what, cudaError_t e) {
-        phf::set_error(PHF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
-        st = PHF_ERR_CUDA;
-    };
-    cudaError_t e;
-    if ((e = cudaMalloc(&dg, ns * MM * sizeof(phf::zc))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dr, ns * MM * sizeof(phf::zc))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dG, MM * sizeof(phf::zc))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dcg, nterm * sizeof(phf::zc))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dcr, nterm * sizeof(phf::zc))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dslot, nterm * sizeof(long long))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st && (e = cudaMalloc(&dcj, nterm * sizeof(int))) != cudaSuccess) fail("cudaMalloc", e);
-    if (!st) {
-        cudaMemcpy(dg, gradmat, ns * MM * sizeof(phf::zc), cudaMemcpyHostToDevice);
-        cudaMemcpy(dr, rdmmat, ns * MM * sizeof(phf::zc), cudaMemcpyHostToDevice);
-        cudaMemcpy(dcg, cg.data(), nterm * sizeof(phf::zc), cudaMemcpyHostToDevice);
-        cudaMemcpy(dcr, cr.data(), nterm * sizeof(phf::zc), cudaMemcpyHostToDevice);
-        cudaMemcpy(dslot, slot.data(), nterm * sizeof(long long), cudaMemcpyHostToDevice);
-        cudaMemcpy(dcj, cj.data(), nterm * sizeof(int), cudaMemcpyHostToDevice);
-        st = phf::launch_localg((int)MM, nterm, dcg, dcr, dslot, dcj, dg, dr, ns, phf::zc{e0.re, e0.im},
-                                phf::zc{ovlp.real(), ovlp.imag()}, dG, 0);
-        if (!st && (e = cudaMemcpy(g, dG, MM * sizeof(phf::zc), cudaMemcpyDeviceToHost)) != cudaSuccess)
-            fail("cudaMemcpy", e);
-    }
-    cudaFree(dg);
-    cudaFree(dr);
-    cudaFree(dG);
-    cudaFree(dcg);
-    cudaFree(dcr);
-    cudaFree(dslot);
-    cudaFree(dcj);
-    return st;
+    PHF_TRY(ar.alloc(&dg, ns * MM));
+    PHF_TRY(ar.alloc(&dr, ns * MM));
+    PHF_TRY(ar.alloc(&dG, MM));
+    PHF_TRY(ar.alloc(&dcg, nterm));
+    PHF_TRY(ar.alloc(&dcr, nterm));
+    PHF_TRY(ar.alloc(&dslot, nterm));
+    PHF_TRY(ar.alloc(&dcj, nterm));
+    PHF_CUDA(cudaMemcpy(dg, gradmat, ns * MM * sizeof(phf::zc), cudaMemcpyHostToDevice));
+    PHF_CUDA(cudaMemcpy(dr, rdmmat, ns * MM * sizeof(phf::zc), cudaMemcpyHostToDevice));
+    PHF_CUDA(cudaMemcpy(dcg, cg.data(), nterm * sizeof(phf::zc), cudaMemcpyHostToDevice));
+    PHF_CUDA(cudaMemcpy(dcr, cr.data(), nterm * sizeof(phf::zc), cudaMemcpyHostToDevice));
+    PHF_CUDA(cudaMemcpy(dslot, slot.data(), nterm * sizeof(long long), cudaMemcpyHostToDevice));
+    PHF_CUDA(cudaMemcpy(dcj, cj.data(), nterm * sizeof(int), cudaMemcpyHostToDevice));
+    PHF_TRY(phf::launch_localg((int)MM, nterm, dcg, dcr, dslot, dcj, dg, dr, ns, phf::zc{e0.re, e0.im},
+                               phf::zc{ovlp.real(), ovlp.imag()}, dG, 0));
+    PHF_CUDA(cudaMemcpy(g, dG, MM * sizeof(phf::zc), cudaMemcpyDeviceToHost));
+    return PHF_OK;
 }
 
 int phf_plan_create(const phf_plan_desc *desc, phf_plan **plan) {

@@ -99,6 +99,65 @@ int profile_read(int c, double *ms, unsigned long long *count) {
     return PHF_OK;
 }
 
+// ---------------------------------------------------------------- memory of one-shot calls
+namespace {
+constexpr size_t kPoolKeep = (size_t)16 << 30;
+constexpr int kPoolDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[kPoolDevices] = {};  // one per device, created at first use, kept until exit
+
+cudaMemPool_t current_pool(bool create) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pools[dev] && create) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        unsigned long long keep = kPoolKeep;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        g_pools[dev] = pool;
+    }
+    return g_pools[dev];
+}
+}  // namespace
+
+cudaError_t pool_alloc(void **p, size_t bytes) {
+    cudaMemPool_t pool = current_pool(true);
+    if (!pool) return cudaErrorMemoryAllocation;
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, 0);
+    if (e == cudaErrorMemoryAllocation) {  // give back what is kept and try once more
+        cudaGetLastError();
+        cudaStreamSynchronize(0);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, 0);
+    }
+    return e;
+}
+
+void pool_free(void *p) { cudaFreeAsync(p, 0); }
+
+void pool_trim() {
+    cudaMemPool_t pool = current_pool(false);
+    size_t fr = 0, tot = 0;
+    if (!pool || cudaMemGetInfo(&fr, &tot) != cudaSuccess) return;
+    unsigned long long held = 0, used = 0;
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held);
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    // keep at most half of what would be free without the kept part
+    const size_t keep = std::min(kPoolKeep, (fr + (size_t)(held - used)) / 2);
+    if (held - used > keep) {
+        cudaStreamSynchronize(0);
+        cudaMemPoolTrimTo(pool, (size_t)used + keep);
+    }
+}
+
 static thread_local std::string t_last_error;
 static thread_local int t_last_status = PHF_OK;
 
@@ -293,11 +352,13 @@ bool cholesky_symmetric(const phf_plan_desc *d) {
 }
 }  // namespace
 
-int plan_create(const phf_plan_desc *d, phf_plan **out) {
+int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
     *out = nullptr;
     PHF_TRY(validate(d));
     auto P = std::make_unique<phf_plan>();
     PlanImpl &p = P->impl;
+    p.arena.pooled = one_shot;
+    p.graphs_ok = !one_shot;  // a graph captured for one evaluation costs more than its launches
     PHF_TRY(check_device(&p.device));
     p.chol = d->nchol > 0;
     p.M = d->nso;
@@ -566,11 +627,11 @@ int plan_create(const phf_plan_desc *d, phf_plan **out) {
         PHF_TRY(upload(p.H1, h1));
         zc *h2 = nullptr;
         PHF_TRY(p.arena.alloc(&p.H2r, MM * MM));
-        PHF_CUDA(cudaMalloc(&h2, MM * MM * sizeof(zc)));
+        PHF_TRY(p.arena.alloc(&h2, MM * MM));
         cudaError_t e = cudaMemcpy(h2, d->htwo, MM * MM * sizeof(zc), cudaMemcpyHostToDevice);
         int st = (e == cudaSuccess) ? launch_permute_h2(M, h2, p.H2r, 0) : PHF_ERR_CUDA;
-        if (e == cudaSuccess && st == PHF_OK) e = cudaDeviceSynchronize();
-        cudaFree(h2);
+        if (e == cudaSuccess && st == PHF_OK) e = cudaStreamSynchronize(0);
+        p.arena.free_one(h2);
         if (e != cudaSuccess) {
             set_error(PHF_ERR_CUDA, std::string("uploading HTwo: ") + cudaGetErrorString(e));
             return PHF_ERR_CUDA;
