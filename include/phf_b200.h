@@ -239,14 +239,14 @@ int phf_plan_eval_device_async(phf_plan *plan, const phf_complex *d_c, phf_compl
 
 /* Batched evaluation of independent instances (the many-instance workload of uneven orbital
  * counts): plans[i] evaluates determinant d_c[i] into d_hs[i], d_yg[i], d_yr[i] exactly as
- * phf_plan_eval_device.  All instances run as one CUDA graph on `stream`, captured on first use
- * for this set of plans and buffers (again after any plan is destroyed or a buffer changes) with
- * the instances spread over 4, 8 or 16 concurrent branches -- the count that timed fastest when the
- * set was captured.  Synchronous; returns the first failing instance's status.  No counterpart in
+ * phf_plan_eval_device.  The instances are spread over up to 16 concurrent branches of `stream`:
+ * launched directly the first time a set of plans and buffers comes, captured as one CUDA graph
+ * when it comes again in the next call, and replayed from then on (anew after any plan is
+ * destroyed or a buffer changes).  Synchronous; returns the first failing instance's status.  No counterpart in
  * the reference (its driver runs one PHF instance at a time). */
 int phf_eval_batch(phf_plan *const *plans, int count, const phf_complex *const *d_c, phf_complex *const *d_hs,
                    phf_complex *const *d_yg, phf_complex *const *d_yr, void *stream);
-/* Concurrent branches of the batch graph phf_eval_batch captured last (0 before any). */
+/* Concurrent branches of the last phf_eval_batch (0 before any). */
 int phf_batch_branches(void);
 
 /* Grid points per pipeline chunk chosen by the plan, and its device workspace in bytes. */

@@ -1852,25 +1852,35 @@ __global__ void gather_flags_kernel(int *const *ptrs, int n, int *out) {
 
 constexpr int kMaxBranches = 16;
 
-// One cached batch graph: the launch sequences of all instances, spread over `branches`
-// concurrent streams, then one kernel copying every plan's status words into `d_flags`.
+// The set of plans and buffers of the last batch, its graph if it was captured, and the status words' buffers (kept
+// for later sets that fit).
 struct BatchGraph {
-    std::vector<const void *> key;  // plans and buffers the graph was captured for
+    std::vector<const void *> key;  // plans and buffers
     unsigned long long epoch = 0;
-    int device = -1, count = 0, branches = 0;
+    int device = -1, branches = 0, cap = 0;
     cudaGraphExec_t exec = nullptr;
     unsigned long long launches = 0;
     int *d_flags = nullptr;   // 2 per plan: overlap status, tensor-core pipeline status
     int **d_ptrs = nullptr;   // where those live
+    std::vector<int *> h_ptrs;
     std::vector<int> h_flags;
-    void release() {
+    void drop() {
         if (exec) cudaGraphExecDestroy(exec);
+        exec = nullptr;
+        key.clear();
+    }
+    int reserve(int count, int dev) {
+        if (cap >= count && device == dev) return PHF_OK;
         if (d_flags) cudaFree(d_flags);
         if (d_ptrs) cudaFree(d_ptrs);
-        exec = nullptr;
         d_flags = nullptr;
         d_ptrs = nullptr;
-        key.clear();
+        cap = 0;
+        PHF_CUDA(cudaMalloc(&d_flags, 2 * (size_t)count * sizeof(int)));
+        PHF_CUDA(cudaMalloc(&d_ptrs, 2 * (size_t)count * sizeof(int *)));
+        cap = count;
+        device = dev;
+        return PHF_OK;
     }
 };
 
@@ -1896,31 +1906,44 @@ int batch_streams(int device) {
     return PHF_OK;
 }
 
-// Capture the batch with `nb` branches into *exec (and its kernel count into *nl).
-int capture_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc *const *d_hs, zc *const *d_yg,
-                  zc *const *d_yr, int nb, int **d_ptrs, int *d_flags, cudaGraphExec_t *exec,
-                  unsigned long long *nl) {
-    const unsigned long long l0 = g_launches;
-    PHF_CUDA(cudaStreamBeginCapture(g_bs.cap, cudaStreamCaptureModeRelaxed));
+// The batch's launches over `nb` branches forked from and joined to `root`, then the status words of every plan.
+int enqueue_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc *const *d_hs, zc *const *d_yg,
+                  zc *const *d_yr, int nb, int **d_ptrs, int *d_flags,
+                  cudaStream_t root) {
     int rc = PHF_OK;
-    cudaError_t e = cudaEventRecord(g_bs.fork, g_bs.cap);
+    cudaError_t e = cudaEventRecord(g_bs.fork, root);
     for (int b = 0; b < nb && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(g_bs.br[b], g_bs.fork, 0);
     for (int i = 0; i < count && rc == PHF_OK && e == cudaSuccess; ++i)
         rc = eval_enqueue(*plans[i], d_c[i], d_hs[i], d_yg[i], d_yr[i], g_bs.br[i % nb], true);
     for (int b = 0; b < nb && e == cudaSuccess; ++b) {
         e = cudaEventRecord(g_bs.join[b], g_bs.br[b]);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(g_bs.cap, g_bs.join[b], 0);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(root, g_bs.join[b], 0);
     }
     if (rc == PHF_OK && e == cudaSuccess) {
-        gather_flags_kernel<<<(2 * count + 255) / 256, 256, 0, g_bs.cap>>>(d_ptrs, 2 * count, d_flags);
+        gather_flags_kernel<<<(2 * count + 255) / 256, 256, 0, root>>>(d_ptrs, 2 * count, d_flags);
         ++g_launches;
         e = cudaGetLastError();
     }
+    if (rc == PHF_OK && e != cudaSuccess) {
+        cudaGetLastError();
+        set_error(PHF_ERR_CUDA, std::string("phf_eval_batch: ") + cudaGetErrorString(e));
+        rc = PHF_ERR_CUDA;
+    }
+    return rc;
+}
+
+// Capture the batch into *exec (and its kernel count into *nl).
+int capture_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc *const *d_hs, zc *const *d_yg,
+                  zc *const *d_yr, int nb, int **d_ptrs, int *d_flags,
+                  cudaGraphExec_t *exec, unsigned long long *nl) {
+    const unsigned long long l0 = g_launches;
+    PHF_CUDA(cudaStreamBeginCapture(g_bs.cap, cudaStreamCaptureModeRelaxed));
+    const int rc = enqueue_batch(plans, count, d_c, d_hs, d_yg, d_yr, nb, d_ptrs, d_flags, g_bs.cap);
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(g_bs.cap, &g);
     *nl = g_launches - l0;
     g_launches = l0;
-    if (rc != PHF_OK || e != cudaSuccess || e2 != cudaSuccess || !g) {
+    if (rc != PHF_OK || e2 != cudaSuccess || !g) {
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         if (rc != PHF_OK) return rc;
@@ -1944,9 +1967,11 @@ void plan_destroyed() {
     ++g_plan_epoch;
 }
 
-// All instances of a batch as one CUDA graph (captured for this set of plans and buffers on first
-// use and replayed after).  The number of concurrent branches is tuned once per captured set:
-// 4, 8 and 16 branches are each captured and timed over one replay, and the fastest is kept.
+// All instances of a batch over concurrent branches: the first call for a set of plans and buffers launches them
+// directly, the next one for the same set captures a CUDA graph, which later calls replay.  16 branches: 16
+// instances of n = 16..96 take 23.8 ms direct and 23.6 replayed with 4, 8 or 16 (27.7 with one), 32 instances of
+// n = 4..14 replay in 3.19, 2.79 and 2.66 ms and run directly in 4.3; capturing and timing the three counts for
+// every set made two alternating sets cost 182 ms a call.
 int plan_eval_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc *const *d_hs, zc *const *d_yg,
                     zc *const *d_yr, cudaStream_t st) {
     if (count <= 0) return PHF_OK;
@@ -1980,60 +2005,42 @@ int plan_eval_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc 
         key.push_back(d_yr[i]);
     }
     BatchGraph &bg = g_batch;
-    if (!(bg.exec && bg.key == key && bg.epoch == g_plan_epoch && bg.device == dev)) {
+    if (!(bg.key == key && bg.epoch == g_plan_epoch && bg.device == dev)) {
         // plans created with autotune are tuned (one direct evaluation each) before the batch is captured
         for (int i = 0; i < count; ++i)
             if (plans[i]->autotune && !plans[i]->tuned) {
                 PHF_TRY(eval_enqueue(*plans[i], d_c[i], d_hs[i], d_yg[i], d_yr[i], st, false));
                 PHF_TRY(read_flag(*plans[i], st));
             }
-        bg.release();
+        bg.drop();
         PHF_TRY(batch_streams(dev));
-        PHF_CUDA(cudaMalloc(&bg.d_flags, 2 * (size_t)count * sizeof(int)));
-        PHF_CUDA(cudaMalloc(&bg.d_ptrs, 2 * (size_t)count * sizeof(int *)));
-        std::vector<int *> ptrs(2 * (size_t)count);
+        PHF_TRY(bg.reserve(count, dev));
+        bg.h_ptrs.resize(2 * (size_t)count);
         for (int i = 0; i < count; ++i) {
-            ptrs[2 * i] = plans[i]->flag;
-            ptrs[2 * i + 1] = plans[i]->ozerr;
+            bg.h_ptrs[2 * i] = plans[i]->flag;
+            bg.h_ptrs[2 * i + 1] = plans[i]->ozerr;
         }
-        PHF_CUDA(cudaMemcpy(bg.d_ptrs, ptrs.data(), ptrs.size() * sizeof(int *), cudaMemcpyHostToDevice));
-        float best = 0.f;
-        for (int nb : {4, 8, 16}) {
-            if (nb > 4 && nb > count) break;
-            const int use = std::min(nb, count);
-            cudaGraphExec_t ex = nullptr;
-            unsigned long long nl = 0;
-            PHF_TRY(capture_batch(plans, count, d_c, d_hs, d_yg, d_yr, use, bg.d_ptrs, bg.d_flags, &ex, &nl));
-            cudaEvent_t e0, e1;
-            PHF_CUDA(cudaEventCreate(&e0));
-            PHF_CUDA(cudaEventCreate(&e1));
-            PHF_CUDA(cudaGraphLaunch(ex, st));  // warm
-            PHF_CUDA(cudaEventRecord(e0, st));
-            PHF_CUDA(cudaGraphLaunch(ex, st));
-            PHF_CUDA(cudaEventRecord(e1, st));
-            PHF_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            PHF_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            if (!bg.exec || ms < best) {
-                if (bg.exec) cudaGraphExecDestroy(bg.exec);
-                bg.exec = ex;
-                bg.branches = use;
-                bg.launches = nl;
-                best = ms;
-            } else {
-                cudaGraphExecDestroy(ex);
-            }
+        PHF_CUDA(cudaMemcpyAsync(bg.d_ptrs, bg.h_ptrs.data(), bg.h_ptrs.size() * sizeof(int *),
+                                 cudaMemcpyHostToDevice, st));
+        bg.branches = std::min(kMaxBranches, count);
+        bg.h_flags.assign(2 * (size_t)count, 0);
+        const int rc = enqueue_batch(plans, count, d_c, d_hs, d_yg, d_yr, bg.branches, bg.d_ptrs, bg.d_flags,
+                                     st);
+        if (rc != PHF_OK) {
+            cudaStreamSynchronize(st);
+            cudaGetLastError();
+            return rc;
         }
-        bg.key = key;
+        bg.key = std::move(key);
         bg.epoch = g_plan_epoch;
         bg.device = dev;
-        bg.count = count;
-        bg.h_flags.assign(2 * (size_t)count, 0);
+    } else {
+        if (!bg.exec)
+            PHF_TRY(capture_batch(plans, count, d_c, d_hs, d_yg, d_yr, bg.branches, bg.d_ptrs, bg.d_flags,
+                                  &bg.exec, &bg.launches));
+        PHF_CUDA(cudaGraphLaunch(bg.exec, st));
+        g_launches += bg.launches;
     }
-    PHF_CUDA(cudaGraphLaunch(bg.exec, st));
-    g_launches += bg.launches;
     PHF_CUDA(cudaMemcpyAsync(bg.h_flags.data(), bg.d_flags, bg.h_flags.size() * sizeof(int), cudaMemcpyDeviceToHost,
                              st));
     PHF_CUDA(cudaStreamSynchronize(st));

@@ -411,7 +411,7 @@ int buildsc_run(phf_complex c0, const phf_complex *c1, const phf_complex *c2, in
 int plan_eval_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc *const *d_hs, zc *const *d_yg,
                     zc *const *d_yr, cudaStream_t st);
 void plan_destroyed();  // invalidates cached batch graphs
-int batch_branches();   // concurrent branches of the last captured batch graph
+int batch_branches();   // concurrent branches of the last batch
 int profile_enable(int on);
 int profile_read(int cls, double *ms, unsigned long long *count);
 int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot = false);  // one_shot: pool memory, no graphs
