@@ -1,6 +1,6 @@
 // Batched FP64 complex inverse, determinant and log-determinant of the rotated overlaps
-// S_w = bra^H R_w ket (N x N): one warp per grid point for N <= 32, else one CTA of 32 x 32 threads
-// per grid point, the matrix resident in shared memory.
+// S_w = bra^H R_w ket (N x N): one warp per grid point for N <= 32, one CTA with the matrix in registers
+// for N <= 100, else one CTA of 32 x 32 threads with the matrix in shared memory.
 //
 // Replaces InvertC (ZGETRF + ZGETRI) and determinantC (ZGETRF) of PHF_fort/Wrappers.f90:195-336
 // as called from RDM (PHF_fort/PHFTools.f90:259-260).  Algorithm: in-place Gauss-Jordan
@@ -12,16 +12,41 @@
 // A zero pivot is reported as status 1 (the reference STOPs "Error in ZGetRF"); a
 // non-finite entry as status 2.  Both are OR-ed into *flag and the outputs of that grid
 // point are zeroed.
+#include <type_traits>
+
 #include "phf_common.cuh"
 
 namespace phf {
 
 namespace {
 
-// One CTA of 32 x 32 threads per grid point (N > 32): thread (ty, tx) updates the elements of rows
+// x - c r, two fused multiply-adds a component
+__device__ __forceinline__ zc submul(zc x, zc c, zc r) {
+    return mkz(fma(c.y, r.y, fma(-c.x, r.x, x.x)), fma(-c.y, r.x, fma(-c.x, r.y, x.y)));
+}
+
+// det = (-1)^{#interchanges} prod(pivots) and log det from log|pivot| and arg(pivot) (plog), the product and the sums
+// taken in pivot order by one thread
+__device__ void write_det(int N, const zc *pivs, const zc *plog, int nswap, zc *det, zc *logdet) {
+    zc d = mkz(1.0, 0.0);
+    double logabs = 0.0, phase = 0.0;
+    for (int k = 0; k < N; ++k) {
+        d = d * pivs[k];
+        logabs += plog[k].x;
+        phase += plog[k].y;
+    }
+    if (nswap & 1) d = mkz(-d.x, -d.y);
+    *det = d;
+    const double pi = 3.14159265358979323846;
+    double ph = fmod(phase + pi * (nswap & 1), 2.0 * pi);
+    if (ph > pi) ph -= 2.0 * pi;
+    if (ph <= -pi) ph += 2.0 * pi;
+    *logdet = mkz(logabs, ph);
+}
+
+// One CTA of 32 x 32 threads per grid point (N > 100): thread (ty, tx) updates the elements of rows
 // ty + 32 m and columns tx + 32 q, so a Gauss-Jordan step is four barriers -- the pivot search is one
-// warp's shuffle arg-max -- and no index division.  Element updates, pivot choice and the determinant
-// are those of the algorithm above, operation for operation.
+// warp's shuffle arg-max -- and no index division.
 constexpr int GJ_T = 32;  // threads per row and per column of the CTA
 
 __global__ void __launch_bounds__(GJ_T *GJ_T) gj_inverse_kernel(int N, const zc *__restrict__ S, long long s_rs,
@@ -158,15 +183,20 @@ __global__ void __launch_bounds__(GJ_T *GJ_T) gj_inverse_kernel(int N, const zc 
 // 32 < N <= 100: the matrix held in registers.  A CTA of R x C threads (R = ceil(N / MR),
 // C = ceil(N / MC)) per grid point; thread (r, c) keeps the MR x MC elements of rows r + R m and
 // columns c + C q for the whole elimination, so a step reads and writes no matrix element through
-// shared memory: only the pivot column (N values), the scaled pivot row (N values) and one
-// candidate per thread row pass through it, with two barriers per step.
+// shared memory: only the pivot column (N values) and the scaled pivot row (N values) pass through
+// it, with two barriers per step.
 //
 // Rows are not interchanged.  Step k takes as pivot the eligible row p (not pivoted before) of
 // maximal |re| + |im| in column k; ties go to the row that the interchanging form would hold at the
-// lowest position, so the pivot sequence, the interchange count and every element update are those of
-// gj_inverse_kernel (the positions are tracked in shared memory: pos[row], row_at[position]).  With
-// p_k the pivot row of step k, the stored result E satisfies E[p_j][k] = inv(S)[j][p_k], which the
-// write-out undoes: element (row, col) goes to inv(S)[step_of_row[row]][piv_row[col]].
+// lowest position, so the pivot sequence and the interchange count are those of gj_inverse_kernel
+// (every warp tracks the positions in its lanes' registers).  With p_k the pivot row of step k, the
+// stored result E satisfies E[p_j][k] = inv(S)[j][p_k], which the write-out undoes: element (row, col)
+// goes to inv(S)[step_of_row[row]][piv_row[col]].
+// Bound: the serial chain of a step (publish, search, division, row, update).  The search is three warp
+// reductions over the published column in every warp, the update is four multiply-adds an element without
+// selects (the owners clear column k and row p beforehand), log and atan2 of the pivots are taken in parallel:
+// 800 matrices of N = 100 in 1.40 ms against 2.40 with candidates through shared memory, a shuffle search and
+// selects in the update; N = 64, 312 of them 0.22 against 0.38; N = 40, 56 of them 69 against 119 us.
 constexpr int GR_NMAX = 128;  // bound of the shared pivot arrays
 
 template <int MR, int MC, int MAXT, int MINB>
@@ -181,22 +211,19 @@ __global__ void __launch_bounds__(MAXT, MINB)
     // colk alternates between two buffers by step parity: step k's column is still read in the update
     // phase after the second barrier, while the owners of column k + 1 may already publish theirs
     __shared__ zc rowk[GR_NMAX], colk2[2][GR_NMAX], pivs[GR_NMAX];
-    __shared__ int pos[GR_NMAX], row_at[GR_NMAX], step_of_row[GR_NMAX], piv_row[GR_NMAX];
-    __shared__ double cand_v[32];
-    __shared__ int cand_pos[32], cand_row[32];
+    __shared__ int step_of_row[GR_NMAX], piv_row[GR_NMAX];
     __shared__ int s_bad;
 
     const int tid = threadIdx.x, lane = tid & 31;
     const bool own = tid < R * C;
     const int r = own ? tid / C : 0, c = own ? tid - (tid / C) * C : 0;
-    const int nrow = R * MR;
     const long long b = blockIdx.x;
     const zc *Sb = S + b * s_bs;
     if (tid == 0) s_bad = 0;
-    for (int i = tid; i < nrow; i += blockDim.x) {
-        pos[i] = i;
-        row_at[i] = i;
-    }
+    for (int i = tid; i < GR_NMAX; i += blockDim.x) colk2[0][i] = colk2[1][i] = mkz(0.0, 0.0);
+    int pos[GR_NMAX / 32];  // position of row lane + 32 u, kept alike by every warp
+#pragma unroll
+    for (int u = 0; u < GR_NMAX / 32; ++u) pos[u] = lane + 32 * u;
     __syncthreads();
     zc a[MR][MC];
 #pragma unroll
@@ -214,60 +241,50 @@ __global__ void __launch_bounds__(MAXT, MINB)
     __syncthreads();
 
     int nswap = 0;  // kept by thread 0
-    for (int k = 0; k < N && s_bad == 0; ++k) {
+    const int bad0 = s_bad;
+    for (int k = 0; k < N && bad0 == 0; ++k) {
         zc *colk = colk2[k & 1];
-        // (A) the owners of column k (slot q with c + C q == k: one q at most) publish it, then pick
-        // their best eligible row from the published values
-        bool owner = false;
+        // (A) the owners of column k (slot q with c + C q == k: one q at most) publish it and clear their copy, so
+        // that the update below is the same for every column
 #pragma unroll
-        for (int q = 0; q < MC; ++q) {
+        for (int q = 0; q < MC; ++q)
             if (own && c + C * q == k) {
-                owner = true;
 #pragma unroll
-                for (int m = 0; m < MR; ++m) colk[r + R * m] = a[m][q];
-            }
-        }
-        if (owner) {
-            double best = -1.0;
-            int bpos = GR_NMAX, brow = -1;
-            for (int row = r; row < nrow; row += R) {
-                const int ps = pos[row];
-                if (ps >= k) {
-                    const double av = abs1(colk[row]);
-                    if (av > best || (av == best && ps < bpos)) {
-                        best = av;
-                        bpos = ps;
-                        brow = row;
-                    }
+                for (int m = 0; m < MR; ++m) {
+                    colk[r + R * m] = a[m][q];
+                    a[m][q] = mkz(0.0, 0.0);
                 }
             }
-            cand_v[r] = best;
-            cand_pos[r] = bpos;
-            cand_row[r] = brow;
-        }
         __syncthreads();
-        // (B) every warp reduces the R candidates: maximal value, then lowest position
-        double pv = lane < R ? cand_v[lane] : -1.0;
-        int pp = lane < R ? cand_pos[lane] : GR_NMAX;
-        int p = lane < R ? cand_row[lane] : -1;
+        // (B) every warp searches the column: maximal value (a non-negative double orders like its bits), then
+        // lowest position
+        unsigned long long best = 0;
+        unsigned at = ~0u;  // position and row of the lane's best candidate
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, pv, off);
-            const int op = __shfl_xor_sync(0xffffffffu, pp, off);
-            const int orow = __shfl_xor_sync(0xffffffffu, p, off);
-            if (ov > pv || (ov == pv && op < pp)) {
-                pv = ov;
-                pp = op;
-                p = orow;
+        for (int u = 0; u < GR_NMAX / 32; ++u) {
+            const double v = abs1(colk[lane + 32 * u]);
+            const unsigned long long key = (unsigned long long)__double_as_longlong(v);
+            const unsigned pr = (unsigned)pos[u] * GR_NMAX + lane + 32 * u;
+            if (pos[u] >= k && lane + 32 * u < N && v == v && (at == ~0u || key > best || (key == best && pr < at))) {
+                best = key;
+                at = pr;
             }
         }
-        if (!(pv > 0.0)) {  // exactly singular (or NaN pivot): every thread leaves at the same step
-            if (tid == 0) s_bad = (pv == 0.0) ? 1 : 2;
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+        const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
+        at = __reduce_min_sync(0xffffffffu, best == ((unsigned long long)hi << 32 | lo) ? at : ~0u);
+        if ((hi | lo) == 0) {  // exactly singular (or only NaN pivots): every thread leaves at the same step
+            if (tid == 0) s_bad = at == ~0u ? 2 : 1;
             break;
         }
-        const zc piv = colk[p];
-        if (own && r == p % R) {  // the owners of row p write the scaled pivot row
-            const zc inv = divz(mkz(1.0, 0.0), piv);
+        const int p = (int)(at % GR_NMAX), pp = (int)(at / GR_NMAX);
+#pragma unroll
+        for (int u = 0; u < GR_NMAX / 32; ++u) {
+            if (pos[u] == k) pos[u] = pp;
+            if (lane + 32 * u == p) pos[u] = k;
+        }
+        if (own && r == p % R) {  // the owners of row p write the scaled pivot row and clear their copy
+            const zc inv = divz(mkz(1.0, 0.0), colk[p]);
             const int mp = p / R;
 #pragma unroll
             for (int m = 0; m < MR; ++m)
@@ -276,41 +293,27 @@ __global__ void __launch_bounds__(MAXT, MINB)
                     for (int q = 0; q < MC; ++q) {
                         const int col = c + C * q;
                         rowk[col] = (col == k) ? inv : a[m][q] * inv;
+                        a[m][q] = mkz(0.0, 0.0);
                     }
                 }
         }
-        if (tid == 0) {  // pivots (det and log det are formed from them at the end) and the positions
-            pivs[k] = piv;
-            if (pp != k) {
-                ++nswap;
-                const int q = row_at[k];
-                row_at[pp] = q;
-                pos[q] = pp;
-                row_at[k] = p;
-                pos[p] = k;
-            }
+        if (tid == 0) {  // pivots (det and log det are formed from them at the end)
+            pivs[k] = colk[p];
+            nswap += pp != k;
             step_of_row[p] = k;
             piv_row[k] = p;
         }
         __syncthreads();
-        // (C) rank-1 update of the register-resident elements
+        // (C) rank-1 update of the register-resident elements; the cleared pivot row takes the factor -1
         if (own) {
             zc rk[MC];
 #pragma unroll
             for (int q = 0; q < MC; ++q) rk[q] = rowk[c + C * q];
 #pragma unroll
             for (int m = 0; m < MR; ++m) {
-                if (r + R * m == p) {
+                const zc ci = r + R * m == p ? mkz(-1.0, 0.0) : colk[r + R * m];
 #pragma unroll
-                    for (int q = 0; q < MC; ++q) a[m][q] = rk[q];
-                } else {
-                    const zc ci = colk[r + R * m];
-#pragma unroll
-                    for (int q = 0; q < MC; ++q) {
-                        const zc x = (c + C * q == k) ? mkz(0.0, 0.0) : a[m][q];
-                        a[m][q] = x - ci * rk[q];
-                    }
-                }
+                for (int q = 0; q < MC; ++q) a[m][q] = submul(a[m][q], ci, rk[q]);
             }
         }
     }
@@ -331,187 +334,130 @@ __global__ void __launch_bounds__(MAXT, MINB)
                 }
             }
     }
+    if (!bad && tid < N) rowk[tid] = mkz(log(hypot(pivs[tid].x, pivs[tid].y)), atan2(pivs[tid].y, pivs[tid].x));
+    __syncthreads();
     if (tid == 0) {
         if (bad) {
             det[b] = mkz(0.0, 0.0);
             logdet[b] = mkz(-INFINITY, 0.0);
             atomicOr(flag, bad);
         } else {
-            // det = (-1)^{#interchanges} prod(pivots), the product and sums taken in pivot order
-            zc d = mkz(1.0, 0.0);
-            double logabs = 0.0, phase = 0.0;
-            for (int k = 0; k < N; ++k) {
-                const zc piv = pivs[k];
-                d = d * piv;
-                logabs += log(hypot(piv.x, piv.y));
-                phase += atan2(piv.y, piv.x);
-            }
-            if (nswap & 1) d = mkz(-d.x, -d.y);
-            det[b] = d;
-            const double pi = 3.14159265358979323846;
-            double ph = fmod(phase + pi * (nswap & 1), 2.0 * pi);
-            if (ph > pi) ph -= 2.0 * pi;
-            if (ph <= -pi) ph += 2.0 * pi;
-            logdet[b] = mkz(logabs, ph);
+            write_det(N, pivs, rowk, nswap, det + b, logdet + b);
         }
     }
 }
 
-// N <= 32: one warp per matrix (lane j owns column j), four matrices per CTA.  The same
-// Gauss-Jordan steps as gj_inverse_kernel -- pivot = first index of the largest |re| + |im| in rows
-// k..N-1 of column k, identical element updates -- but warp-synchronous: the pivot search is a
-// shuffle arg-max and the steps are separated by __syncwarp only.  The pivots are kept and lane 0
-// forms det and log det from them at the end, in pivot order.
-constexpr int WI_WARPS = 4, WI_P = 33;  // matrices per CTA, row pitch (complex) of the shared copy
+// N <= 32: one warp per matrix, lane j holding column j in registers, padded to NB rows (a multiple of four).  The
+// same Gauss-Jordan steps with the rows rotated by one register per step: step k's row is always register 0, the
+// rows below it follow, the finished rows come last, so every register index is a constant of the unrolled code.
+// Lane k passes its column through shared memory; lane i takes candidate i of the pivot search, an arg-max by
+// three warp reductions (a non-negative double orders like its bits).  The column interchanges at the end are
+// a permutation of the lanes' store addresses.
+// Bound: the serial chain of a step (search, division, update).  Measured with the launch and status read: 800
+// matrices of N = 32 in 82 us against 134 with the matrix in shared memory, a shuffle search and log and atan2
+// by one lane (1650 warp instructions a step); 260 of N = 24 in 47 against 84; 112 of N = 10 in 33 against 46.
+constexpr int WI_WARPS = 4;  // matrices per CTA
 
-__host__ __device__ constexpr size_t wi_warp_bytes() { return (size_t)(32 * WI_P + 64) * sizeof(zc) + 32 * sizeof(int); }
-
+template <int NB>
 __global__ void __launch_bounds__(WI_WARPS * 32) gj_inverse_warp_kernel(
     int N, int batch, const zc *__restrict__ S, long long s_rs, long long s_bs, zc *__restrict__ Sinv, long long i_rs,
     long long i_bs, zc *__restrict__ det, zc *__restrict__ logdet, int *__restrict__ flag) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ zc s_col[WI_WARPS][NB], s_piv[WI_WARPS][NB], s_log[WI_WARPS][NB];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long b = (long long)blockIdx.x * WI_WARPS + warp;
     if (b >= batch) return;  // the whole warp leaves; nothing below synchronises beyond the warp
-    unsigned char *base = smem_raw + (size_t)warp * wi_warp_bytes();
-    zc *A = reinterpret_cast<zc *>(base);  // N x N, row i at A + i WI_P
-    zc *colk = A + 32 * WI_P;              // saved column k
-    zc *pivs = colk + 32;                  // pivots in order
-    int *perm = reinterpret_cast<int *>(pivs + 32);
+    zc *colk = s_col[warp], *pivs = s_piv[warp], *plog = s_log[warp];
     const unsigned full = 0xffffffffu;
     const bool own = lane < N;
 
     const zc *Sb = S + b * s_bs;
     int bad = 0;
-    if (own) {
-        for (int i0 = 0; i0 < N; i0 += 8) {  // eight global loads in flight, then the shared stores
-            zc v[8];
+    zc a[NB];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (i0 + u < N) v[u] = Sb[(long long)(i0 + u) * s_rs + lane];
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (i0 + u < N) {
-                    if (!isfinite(v[u].x) || !isfinite(v[u].y)) bad = 2;
-                    A[(i0 + u) * WI_P + lane] = v[u];
-                }
-        }
+    for (int i = 0; i < NB; ++i) {
+        a[i] = mkz(0.0, 0.0);
+        if (own && i < N) a[i] = Sb[(long long)i * s_rs + lane];
     }
-    bad = __reduce_max_sync(full, bad);
-    __syncwarp();
-
-    for (int k = 0; k < N && bad == 0; ++k) {
-        double a = -1.0;
-        int idx = N;
-        if (lane >= k && lane < N) {
-            const double v = abs1(A[lane * WI_P + k]);
-            if (v > a) {  // NaN never becomes a candidate
-                a = v;
-                idx = lane;
-            }
-        }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double oa = __shfl_xor_sync(full, a, off);
-            const int oi = __shfl_xor_sync(full, idx, off);
-            if (oa > a || (oa == a && oi < idx)) {
-                a = oa;
-                idx = oi;
-            }
+    for (int i = 0; i < NB; ++i)
+        if (!isfinite(a[i].x) || !isfinite(a[i].y)) bad = 2;
+    bad = __reduce_max_sync(full, bad);
+
+    int nswap = 0, my_perm = 0;  // lane k keeps the row interchanged with row k
+    for (int k = 0; k < N && bad == 0; ++k) {
+        if (lane == k) {
+#pragma unroll
+            for (int i = 0; i < NB; ++i) colk[i] = a[i];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) a[i] = mkz(0.0, 0.0);
         }
-        const int p = idx;
-        if (!(a > 0.0)) {  // exactly singular (or NaN pivot)
-            bad = (a == 0.0) ? 1 : 2;
+        __syncwarp();
+        unsigned long long key = 0;
+        bool cand = false;  // NaN never becomes a candidate
+        if (lane < N - k) {
+            const double v = abs1(colk[lane]);
+            cand = v == v;
+            if (cand) key = (unsigned long long)__double_as_longlong(v);
+        }
+        const unsigned hi = __reduce_max_sync(full, (unsigned)(key >> 32));
+        const unsigned lo = __reduce_max_sync(full, (unsigned)(key >> 32) == hi ? (unsigned)key : 0u);
+        const unsigned who = __ballot_sync(full, cand && key == ((unsigned long long)hi << 32 | lo));
+        if ((hi | lo) == 0) {  // exactly singular (or only NaN pivots)
+            bad = who ? 1 : 2;
             break;
         }
-        if (p != k && own) {
-            const zc t = A[k * WI_P + lane];
-            A[k * WI_P + lane] = A[p * WI_P + lane];
-            A[p * WI_P + lane] = t;
-        }
-        __syncwarp();
-        const zc piv = A[k * WI_P + k];
-        const zc inv = divz(mkz(1.0, 0.0), piv);
-        zc rk = mkz(0.0, 0.0);
-        if (own) {
-            rk = (lane == k) ? inv : A[k * WI_P + lane] * inv;
-            colk[lane] = A[lane * WI_P + k];
-        }
-        if (lane == 0) {
-            pivs[k] = piv;
-            perm[k] = p;
-        }
-        __syncwarp();
-        if (own) {  // rows in batches of eight: loads, then arithmetic, then stores (latencies overlap)
-            for (int i0 = 0; i0 < N; i0 += 8) {
-                zc av[8], cv[8];
+        const int p = __ffs(who) - 1;
+        const zc piv = colk[p];
+        if (lane == k) my_perm = k + p;
+        if (p != 0) {
+            ++nswap;
+            const zc c0 = colk[0], r0 = a[0];
+            __syncwarp();
+            if (lane == 0) colk[p] = c0;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int i = i0 + u;
-                    if (i < N) {
-                        av[u] = A[i * WI_P + lane];
-                        cv[u] = colk[i];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int i = i0 + u;
-                    if (i < N) {
-                        if (i == k) {
-                            av[u] = rk;
-                        } else {
-                            const zc x = (lane == k) ? mkz(0.0, 0.0) : av[u];
-                            av[u] = x - cv[u] * rk;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (i0 + u < N) A[(i0 + u) * WI_P + lane] = av[u];
-            }
-        }
-        __syncwarp();
-    }
-    if (bad == 0) {
-        // undo the row interchanges as column interchanges, in reverse order (lane i swaps row i)
-        for (int k = N - 1; k >= 0; --k) {
-            const int p = perm[k];
-            if (p != k && own) {
-                const zc t = A[lane * WI_P + k];
-                A[lane * WI_P + k] = A[lane * WI_P + p];
-                A[lane * WI_P + p] = t;
+            for (int i = 1; i < NB; ++i) {
+                const bool h = i == p;
+                const zc t = a[i];
+                a[i] = mkz(h ? r0.x : t.x, h ? r0.y : t.y);
+                a[0] = mkz(h ? t.x : a[0].x, h ? t.y : a[0].y);
             }
             __syncwarp();
         }
+        if (lane == 0) pivs[k] = piv;
+        const zc inv = divz(mkz(1.0, 0.0), piv);
+        const zc rk = lane == k ? inv : a[0] * inv;
+#pragma unroll
+        for (int i = 1; i < NB; ++i) {
+            if (i % 8 == 0) __syncwarp();  // bounds how far ahead the column is loaded (registers)
+            a[i - 1] = submul(a[i], colk[i], rk);
+        }
+        a[NB - 1] = rk;
+        __syncwarp();
+    }
+    // undo the row interchanges as column interchanges, in reverse order: where the lane's column ends up
+    int col = lane;
+    for (int k = N - 1; k >= 0; --k) {
+        const int p = __shfl_sync(full, my_perm, k);
+        col = col == k ? p : (col == p ? k : col);
     }
     zc *Ib = Sinv + b * i_bs;
-    for (int i = 0; i < N; ++i)
-        if (own) Ib[(long long)i * i_rs + lane] = bad ? mkz(0.0, 0.0) : A[i * WI_P + lane];
+    if (bad) {
+        for (int i = 0; i < N; ++i)
+            if (own) Ib[(long long)i * i_rs + lane] = mkz(0.0, 0.0);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NB; ++i)  // register i holds row i - (NB - N)
+            if (own && i >= NB - N) Ib[(long long)(i - (NB - N)) * i_rs + col] = a[i];
+        if (own) plog[lane] = mkz(log(hypot(pivs[lane].x, pivs[lane].y)), atan2(pivs[lane].y, pivs[lane].x));
+    }
+    __syncwarp();
     if (lane == 0) {
         if (bad) {
             det[b] = mkz(0.0, 0.0);
             logdet[b] = mkz(-INFINITY, 0.0);
             atomicOr(flag, bad);
         } else {
-            zc d = mkz(1.0, 0.0);
-            double logabs = 0.0, phase = 0.0;
-            int nswap = 0;
-            for (int k = 0; k < N; ++k) {
-                const zc piv = pivs[k];
-                d = d * piv;
-                logabs += log(hypot(piv.x, piv.y));
-                phase += atan2(piv.y, piv.x);
-                if (perm[k] != k) {
-                    d = mkz(-d.x, -d.y);
-                    ++nswap;
-                }
-            }
-            det[b] = d;
-            const double pi = 3.14159265358979323846;
-            double ph = fmod(phase + pi * (nswap & 1), 2.0 * pi);
-            if (ph > pi) ph -= 2.0 * pi;
-            if (ph <= -pi) ph += 2.0 * pi;
-            logdet[b] = mkz(logabs, ph);
+            write_det(N, pivs, plog, nswap, det + b, logdet + b);
         }
     }
 }
@@ -523,11 +469,22 @@ size_t overlap_inverse_smem(int N) { return (size_t)N * N * sizeof(zc) + 2 * (si
 int overlap_inverse(int N, int batch, const zc *S, long long s_rs, long long s_bs, zc *Sinv, long long i_rs,
                     long long i_bs, zc *det, zc *logdet, int *flag, cudaStream_t st) {
     if (N <= 32) {
-        const size_t smem = WI_WARPS * wi_warp_bytes();
-        PHF_CUDA(cudaFuncSetAttribute(gj_inverse_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         ProfScope prof(st, PROF_INVERSE);
-        gj_inverse_warp_kernel<<<(unsigned)((batch + WI_WARPS - 1) / WI_WARPS), WI_WARPS * 32, smem, st>>>(
-            N, batch, S, s_rs, s_bs, Sinv, i_rs, i_bs, det, logdet, flag);
+        const unsigned grid = (unsigned)((batch + WI_WARPS - 1) / WI_WARPS);
+        const auto launch = [&](auto nb) {
+            gj_inverse_warp_kernel<nb.value><<<grid, WI_WARPS * 32, 0, st>>>(N, batch, S, s_rs, s_bs, Sinv, i_rs, i_bs,
+                                                                            det, logdet, flag);
+        };
+        switch ((N + 3) / 4) {
+            case 1: launch(std::integral_constant<int, 4>{}); break;
+            case 2: launch(std::integral_constant<int, 8>{}); break;
+            case 3: launch(std::integral_constant<int, 12>{}); break;
+            case 4: launch(std::integral_constant<int, 16>{}); break;
+            case 5: launch(std::integral_constant<int, 20>{}); break;
+            case 6: launch(std::integral_constant<int, 24>{}); break;
+            case 7: launch(std::integral_constant<int, 28>{}); break;
+            default: launch(std::integral_constant<int, 32>{}); break;
+        }
         ++g_launches;
         PHF_CHECK_LAUNCH();
         return PHF_OK;
