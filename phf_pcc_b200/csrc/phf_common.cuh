@@ -35,6 +35,10 @@ __host__ __device__ __forceinline__ zc divz(zc a, zc b) {
     }
 }
 
+struct FoldSums {  // accumulated sums and their compensations; the ket side's (K) may be null
+    const zc *G, *cG, *R, *cR, *KG, *cKG, *KR, *cKR, *HS, *cHS;
+};
+
 // ---------------------------------------------------------------- errors
 struct Error {
     int status;

@@ -650,22 +650,28 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
     PHF_TRY(p.arena.alloc(&p.T2, (size_t)p.ny * p.npg * MN));
     if (p.chol) PHF_TRY(p.arena.alloc(&p.V, (size_t)p.L * MN));
     const size_t nslot = (size_t)p.nci * p.nci;
-    PHF_TRY(p.arena.alloc(&p.accG, nslot * MN));
-    PHF_TRY(p.arena.alloc(&p.compG, nslot * MN));
-    PHF_TRY(p.arena.alloc(&p.accR, nslot * MN));
-    PHF_TRY(p.arena.alloc(&p.compR, nslot * MN));
-    PHF_TRY(p.arena.alloc(&p.accHS, 2 * nslot));
-    PHF_TRY(p.arena.alloc(&p.compHS, 2 * nslot));
+    // the accumulators in one buffer, cleared by one launch: the sums, their compensations, the status word
+    p.acc_bytes = ((size_t)(p.exact ? 8 : 4) * nslot * MN + 4 * nslot) * sizeof(zc) + sizeof(int);
+    unsigned char *acc = nullptr;
+    PHF_TRY(p.arena.alloc(&acc, p.acc_bytes));
+    p.accG = reinterpret_cast<zc *>(acc);
+    p.compG = p.accG + nslot * MN;
+    p.accR = p.compG + nslot * MN;
+    p.compR = p.accR + nslot * MN;
+    zc *next = p.compR + nslot * MN;
+    if (p.exact) {
+        p.accKG = next;
+        p.compKG = p.accKG + nslot * MN;
+        p.accKR = p.compKG + nslot * MN;
+        p.compKR = p.accKR + nslot * MN;
+        next = p.compKR + nslot * MN;
+    }
+    p.accHS = next;
+    p.compHS = p.accHS + 2 * nslot;
+    p.flag = reinterpret_cast<int *>(p.compHS + 2 * nslot);
     PHF_TRY(p.arena.alloc(&p.tmpG, MN));
     PHF_TRY(p.arena.alloc(&p.outMM, 2 * nslot * MM));  // every slot's Gradmat and Rdmmat block
     if (p.exact || p.fold_h) PHF_TRY(p.arena.alloc(&p.Hb, MN));
-    if (p.exact) {
-        PHF_TRY(p.arena.alloc(&p.accKG, nslot * MN));
-        PHF_TRY(p.arena.alloc(&p.compKG, nslot * MN));
-        PHF_TRY(p.arena.alloc(&p.accKR, nslot * MN));
-        PHF_TRY(p.arena.alloc(&p.compKR, nslot * MN));
-    }
-    PHF_TRY(p.arena.alloc(&p.flag, 1));
 
     // chunk size from the workspace budget.  The streamed form regenerates its exchange rows once
     // per chunk (2 n^4 L flops against 16 n^4 per point), so by default it takes up to 45 % of the
@@ -735,7 +741,6 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
     PHF_TRY(p.arena.alloc(&p.logdet, p.b));
     PHF_TRY(p.arena.alloc(&p.e1, p.b));
     PHF_TRY(p.arena.alloc(&p.e2, p.b));
-    PHF_TRY(p.arena.alloc(&p.scal, 2 * (size_t)p.b));
     if (p.chol && p.eri) {
         const size_t n2 = (size_t)n * n, b = (size_t)p.b;
         PHF_TRY(p.arena.alloc(&p.Gam, b * MM));
@@ -1378,11 +1383,9 @@ int ket_side(PlanImpl &p, int v, int bc, int w0, cudaStream_t st) {
         std::swap(src, dst);
         std::swap(srcr, dstr);
     }
-    PHF_TRY(launch_scale_conj_det(M, N, bc, p.det, src, ld, st));
-    PHF_TRY(launch_scale_conj_det(M, N, bc, p.det, srcr, ld, st));
     const int nb2 = p.nb * p.nb;
-    PHF_TRY(launch_accumulate(nb2, M, N, bc, p.Wt, p.nomega, w0, p.slotmap + (size_t)v * nb2, src, srcr, ld, nullptr,
-                              p.accKG, p.compKG, p.accKR, p.compKR, nullptr, nullptr, p.acc_scratch, st, 1));
+    PHF_TRY(launch_accumulate(nb2, M, N, bc, p.Wt, p.nomega, w0, p.slotmap + (size_t)v * nb2, src, srcr, ld, p.det,
+                              nullptr, nullptr, p.accKG, p.compKG, p.accKR, p.compKR, nullptr, nullptr, p.acc_scratch, st, 1));
     return PHF_OK;
 }
 
@@ -1480,43 +1483,24 @@ int run_variant(PlanImpl &p, int v, cudaStream_t st) {
                               nullptr, st));
         PHF_TRY(zgemm_strided(M, N, N, bc, 1, ZM1, vz(p.Xs, ld, 1, N), vz(p.W, ld, 1, N), Z1, vo(p.GX, ld, 1, N), nullptr,
                               st));
-        PHF_TRY(launch_epilogue(M, N, bc, p.GX, p.Xs, ld, p.det, p.e1, p.e2, p.scal, st));
         const int nb2 = p.nb * p.nb;
-        PHF_TRY(launch_accumulate(nb2, M, N, bc, p.Wt, p.nomega, w0, p.slotmap + (size_t)v * nb2, p.GX, p.Xs, ld, p.scal,
-                                  p.accG, p.compG, p.accR, p.compR, p.accHS, p.compHS, p.acc_scratch, st));
+        PHF_TRY(launch_accumulate(nb2, M, N, bc, p.Wt, p.nomega, w0, p.slotmap + (size_t)v * nb2, p.GX, p.Xs, ld, p.det,
+                                  p.e1, p.e2, p.accG, p.compG, p.accR, p.compR, p.accHS, p.compHS, p.acc_scratch, st));
         if (p.exact) PHF_TRY(ket_side(p, v, bc, w0, st));
     }
     return PHF_OK;
 }
 
 int zero_acc(PlanImpl &p, cudaStream_t st) {
-    const size_t nslot = (size_t)p.nci * p.nci, MN = (size_t)p.M * p.N;
-    PHF_CUDA(cudaMemsetAsync(p.accG, 0, nslot * MN * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.compG, 0, nslot * MN * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.accR, 0, nslot * MN * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.compR, 0, nslot * MN * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.accHS, 0, 2 * nslot * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.compHS, 0, 2 * nslot * sizeof(zc), st));
-    PHF_CUDA(cudaMemsetAsync(p.flag, 0, sizeof(int), st));
-    if (p.exact) {
-        PHF_CUDA(cudaMemsetAsync(p.accKG, 0, nslot * MN * sizeof(zc), st));
-        PHF_CUDA(cudaMemsetAsync(p.compKG, 0, nslot * MN * sizeof(zc), st));
-        PHF_CUDA(cudaMemsetAsync(p.accKR, 0, nslot * MN * sizeof(zc), st));
-        PHF_CUDA(cudaMemsetAsync(p.compKR, 0, nslot * MN * sizeof(zc), st));
-    }
+    PHF_CUDA(cudaMemsetAsync(p.accG, 0, p.acc_bytes, st));
     return PHF_OK;
 }
 
-int fold_acc(PlanImpl &p, cudaStream_t st) {
-    const long long nslot = (long long)p.nci * p.nci, MN = (long long)p.M * p.N;
-    PHF_TRY(launch_fold_comp(nslot * MN, p.accG, p.compG, st));
-    PHF_TRY(launch_fold_comp(nslot * MN, p.accR, p.compR, st));
-    PHF_TRY(launch_fold_comp(2 * nslot, p.accHS, p.compHS, st));
-    if (p.exact) {
-        PHF_TRY(launch_fold_comp(nslot * MN, p.accKG, p.compKG, st));
-        PHF_TRY(launch_fold_comp(nslot * MN, p.accKR, p.compKR, st));
-    }
-    return PHF_OK;
+// The folded sums into outG, outR, outHS (rows mapped by `rowmap`; averaged with the ket side's sums when `ket`).
+int fold_acc(PlanImpl &p, const int *rowmap, bool ket, zc *outG, zc *outR, zc *outHS, cudaStream_t st) {
+    FoldSums S{p.accG, p.compG, p.accR, p.compR, nullptr, nullptr, nullptr, nullptr, p.accHS, p.compHS};
+    if (ket) S.KG = p.accKG, S.cKG = p.compKG, S.KR = p.accKR, S.cKR = p.compKR;
+    return launch_fold_out(p.nci * p.nci, p.M, p.N, rowmap, S, outG, outR, outHS, st);
 }
 
 // Status of an evaluation from its flag word and the tensor-core GEMM error word (host copies).
@@ -1669,7 +1653,7 @@ int plan_buildhsg(PlanImpl &p, const phf_complex *z, phf_complex *hmat, phf_comp
         }
         PHF_TRY(launch_captured(p, v, st, [&](cudaStream_t s) -> int { return run_variant(p, v, s); }));
     }
-    PHF_TRY(fold_acc(p, st));
+    PHF_TRY(fold_acc(p, nullptr, false, p.accG, p.accR, p.accHS, st));
 
     // Gradmat_a = T Yg_a bra_a^H, Rdmmat likewise (T = Ref^H in the Cholesky form); every block is
     // formed on the device first, then all blocks and H, S come back in one synchronisation
@@ -1776,25 +1760,17 @@ int eval_enqueue(PlanImpl &p, const zc *d_c, zc *d_hs, zc *d_yg, zc *d_yr, cudaS
     const long long MN = (long long)M * N;
     if (p.chol) {
         // rows of C from [alpha; beta] order to the working order: bra[r'] = C[perm[r']]
-        PHF_TRY(launch_permute_rows(M, N, 1, p.permdev, d_c, N, 0, p.bra, 0, st));
+        PHF_TRY(launch_permute_rows(M, N, p.permdev, d_c, p.bra, p.kety, st));
     } else {
         PHF_CUDA(cudaMemcpyAsync(p.bra, d_c, MN * sizeof(zc), cudaMemcpyDeviceToDevice, st));
     }
-    if (p.chol) {
-        PHF_CUDA(cudaMemcpyAsync(p.kety, p.bra, MN * sizeof(zc), cudaMemcpyDeviceToDevice, st));
-    } else {
+    if (!p.chol) {
         // kety = Ref C (reference AO order)
         PHF_TRY(zgemm_strided(M, N, M, 1, 1, Z1, vz(p.Refw, M, 1), vz(p.bra, N, 1), Z0, vo(p.kety, N, 1), nullptr, st));
     }
-    const long long ns = (long long)p.nci * p.nci;
     auto body = [&](cudaStream_t s) -> int {
         PHF_TRY(zero_acc(p, s));
         PHF_TRY(run_variant(p, 0, s));
-        PHF_TRY(fold_acc(p, s));
-        if (p.exact) {  // symmetrised bra + ket derivative
-            PHF_TRY(launch_average(ns * MN, p.accG, p.accKG, p.accG, s));
-            PHF_TRY(launch_average(ns * MN, p.accR, p.accKR, p.accR, s));
-        }
         return PHF_OK;
     };
     if (in_graph) {
@@ -1803,16 +1779,8 @@ int eval_enqueue(PlanImpl &p, const zc *d_c, zc *d_hs, zc *d_yg, zc *d_yr, cudaS
         PHF_TRY(maybe_tune(p, st, body));
         PHF_TRY(launch_captured(p, 4, st, body));
     }
-    PHF_CUDA(cudaMemcpyAsync(d_hs, p.accHS, 2 * ns * sizeof(zc), cudaMemcpyDeviceToDevice, st));
-    if (p.chol) {
-        // back to [alpha; beta] order: out[r] = acc[inv[r]]
-        PHF_TRY(launch_permute_rows(M, N, (int)ns, p.permdev + M, p.accG, N, MN, d_yg, MN, st));
-        PHF_TRY(launch_permute_rows(M, N, (int)ns, p.permdev + M, p.accR, N, MN, d_yr, MN, st));
-    } else {
-        PHF_CUDA(cudaMemcpyAsync(d_yg, p.accG, ns * MN * sizeof(zc), cudaMemcpyDeviceToDevice, st));
-        PHF_CUDA(cudaMemcpyAsync(d_yr, p.accR, ns * MN * sizeof(zc), cudaMemcpyDeviceToDevice, st));
-    }
-    return PHF_OK;
+    // rows back to [alpha; beta] order where they were permuted; symmetrised bra + ket derivative in exact mode
+    return fold_acc(p, p.chol ? p.permdev + M : nullptr, p.exact, d_yg, d_yr, d_hs, st);
 }
 
 int plan_eval_device(PlanImpl &p, const zc *d_c, zc *d_hs, zc *d_yg, zc *d_yr, cudaStream_t st) {

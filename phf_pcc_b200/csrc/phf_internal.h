@@ -125,20 +125,18 @@ int launch_add_coulomb_diag(int n, int b, const double *Jr, long long jrs, long 
                             const double *h = nullptr);
 int launch_spin_block_y(int n, int N, int bc, int w0, int blk, const zc *R1b, const zc *T2, long long ld2, zc *Ys,
                         long long ld, cudaStream_t st);
-int launch_epilogue(int M, int N, int b, zc *G, zc *X, long long ldX, const zc *det, const zc *e1,
-                    const zc *e2, zc *scal, cudaStream_t st);
 size_t accumulate_scratch_bytes(int nslot, int M, int N, int b);
+// e1, e2 null: no energy term (the ket side); accHS null: no scalars
 int launch_accumulate(int nslot, int M, int N, int b, const zc *Wt, long long nomega, long long w0, const int *slotmap,
-                      const zc *G, const zc *R, long long ldX, const zc *scal, zc *accG, zc *compG, zc *accR,
-                      zc *compR, zc *accHS, zc *compHS, void *scratch, cudaStream_t st, int conj_weights = 0);
-int launch_fold_comp(long long n, zc *a, const zc *c, cudaStream_t st);
+                      const zc *G, const zc *R, long long ldX, const zc *det, const zc *e1, const zc *e2, zc *accG,
+                      zc *compG, zc *accR, zc *compR, zc *accHS, zc *compHS, void *scratch, cudaStream_t st,
+                      int conj_weights = 0);
+int launch_fold_out(int nslot, int M, int N, const int *rowmap, const FoldSums &S, zc *outG, zc *outR, zc *outHS,
+                    cudaStream_t st);
 int launch_ket_prep(int M, int N, int b, const zc *Hb, const zc *bra, const zc *e1, const zc *e2, zc *V, long long ld,
                     cudaStream_t st);
-int launch_scale_conj_det(int M, int N, int b, const zc *det, zc *P, long long ld, cudaStream_t st);
-int launch_average(long long n, const zc *a, const zc *b, zc *out, cudaStream_t st);
 int launch_permute_h2(int M, const zc *H2, zc *H2r, cudaStream_t st);
-int launch_permute_rows(int M, int N, int nbatch, const int *rowmap, const zc *in, long long ldin, long long bs_in,
-                        zc *out, long long bs_out, cudaStream_t st);
+int launch_permute_rows(int M, int N, const int *rowmap, const zc *in, zc *out, zc *out2, cudaStream_t st);
 int launch_localg(int MM, int nterm, const zc *coef_g, const zc *coef_r, const long long *slot_of_term,
                   const int *conj_of_term, const zc *gradmat, const zc *rdmmat, long long nslot, zc e0, zc ovlp, zc *G,
                   cudaStream_t st);
@@ -341,11 +339,12 @@ struct PlanImpl {
     int b = 0;
     zc *Ys = nullptr, *Ys2 = nullptr, *S = nullptr, *Sinv = nullptr, *Xs = nullptr, *HX = nullptr, *GX = nullptr,
        *W = nullptr, *T = nullptr, *Q = nullptr, *Pv = nullptr, *Gv = nullptr, *det = nullptr, *logdet = nullptr,
-       *e1 = nullptr, *e2 = nullptr, *e2part = nullptr, *scal = nullptr;
+       *e1 = nullptr, *e2 = nullptr, *e2part = nullptr;
     int *flag = nullptr;
     // accumulators
     zc *accG = nullptr, *compG = nullptr, *accR = nullptr, *compR = nullptr, *accHS = nullptr, *compHS = nullptr;
     zc *tmpG = nullptr, *outMM = nullptr;
+    size_t acc_bytes = 0;              // the accumulators' buffer (accG first)
     void *acc_scratch = nullptr;       // partial sums of the two-stage accumulation
     // ket-side gradient (exact mode)
     zc *Hb = nullptr, *Vk = nullptr, *Pk = nullptr, *Pk2 = nullptr, *Prk = nullptr, *Prk2 = nullptr;

@@ -65,43 +65,28 @@ __global__ void __launch_bounds__(NT) trace_conj_kernel(int M, int N, const zc *
     __shared__ zc sh[NT];
     const long long w = blockIdx.x;
     zc s = mkz(0, 0);
-    for (int e = threadIdx.x; e < M * N; e += NT) {
-        int r = e / N, j = e - r * N;
-        const long long o = (long long)r * ldX + w * N + j;
-        const zc x = X[o];
-        s = s + conjz(C[e]) * x;
-        if (add) X[o] = x + add[o];  // X <- X + add once the trace has read X
+    for (int e0 = threadIdx.x; e0 < M * N; e0 += 4 * NT) {  // four loads in flight, summed in order
+        zc x[4], c[4];
+        long long o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int e = e0 + u * NT;
+            if (e < M * N) {
+                const int r = e / N, j = e - r * N;
+                o[u] = (long long)r * ldX + w * N + j;
+                x[u] = X[o[u]];
+                c[u] = C[e];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (e0 + u * NT < M * N) {
+                s = s + conjz(c[u]) * x[u];
+                if (add) X[o[u]] = x[u] + add[o[u]];  // X <- X + add once the trace has read X
+            }
     }
     s = block_sum(s, sh);
     if (threadIdx.x == 0) out[w] = sub ? scale * s - sub_scale * sub[w] : scale * s;
-}
-
-// Energy/gradient epilogue over a chunk of b grid points (Gradient, PHFTools.f90:291-308, in
-// the rank-N form): with h_w = e1_w + e2_w and N_w = det S_w,
-//   G <- N_w (G + h_w X)          where G already holds HX + GammaX - X W_w
-//   X <- N_w X
-//   scal[2w] = N_w h_w, scal[2w+1] = N_w
-__global__ void __launch_bounds__(NT) epilogue_kernel(int M, int N, int b, zc *G, zc *X, long long ldX,
-                                                      const zc *det, const zc *e1, const zc *e2, zc *scal) {
-    const long long total = (long long)M * b * N;
-    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < total; e += (long long)gridDim.x * NT) {
-        long long r = e / ((long long)b * N);
-        long long c = e - r * ((long long)b * N);
-        int w = (int)(c / N);
-        long long o = r * ldX + c;
-        zc h = e1[w] + e2[w];
-        zc nd = det[w];
-        zc x = X[o];
-        G[o] = nd * (G[o] + h * x);
-        X[o] = nd * x;
-    }
-    if (blockIdx.x == 0) {
-        for (int w = threadIdx.x; w < b; w += NT) {
-            zc h = e1[w] + e2[w];
-            scal[2 * w] = det[w] * h;
-            scal[2 * w + 1] = det[w];
-        }
-    }
 }
 
 // Neumaier compensated add of a complex term into (s, c)
@@ -112,58 +97,69 @@ __device__ __forceinline__ void neumaier(double &s, double &c, double x) {
     s = t;
 }
 
-// Weighted accumulation over a chunk of grid points (PHFTools.f90:137-166):
-//   accG[a] += sum_w Wt[s, w0 + w] * G_w,  accR[a] += sum_w Wt[s, w0 + w] * R_w,
-//   accHS[a] += sum_w Wt[s, w0 + w] * (N h, N)_w      with a = slotmap[s].
+// Weighted accumulation over a chunk of grid points (PHFTools.f90:137-166) with the energy/gradient epilogue
+// (Gradient, PHFTools.f90:291-308, in the rank-N form) applied on the way.  With h_w = e1_w + e2_w, N_w = det S_w
+// and c_w = Wt[s, w0 + w] N_w (both conjugated for the ket side, which has no h: e1 null):
+//   accG[a] += sum_w c_w (G_w + h_w R_w),  accR[a] += sum_w c_w R_w,  accHS[a] += sum_w c_w (h_w, 1)
+// with a = slotmap[s]; G holds HX + GammaX - X W_w, R holds X_w.
 // Two stages with a fixed partition, so the result does not depend on scheduling:
 //   stage 1: thread (element, group q) sums the points [q*ACC_GROUP, (q+1)*ACC_GROUP) in order
-//            with Neumaier compensation into part[q] (sum, compensation);
+//            with Neumaier compensation into part[q] (sum, compensation); the two scalars are element MN;
 //   stage 2: thread (element) adds part[0..ngroups) in order into the running (acc, comp).
-constexpr int ACC_GROUP = 32;
+// Bound: G and R read once; at small sizes the serial chain of the 32 points, so their loads go four ahead and
+// the group's factors come from shared memory (M = 40 to 96 spin orbitals: 34 us as one load after another, after
+// 4 to 9 us of a separate epilogue that wrote G and R again).
+constexpr int ACC_GROUP = 32, ACC_NT = 128;
 
 struct AccPart {
     double gs_r, gs_i, gc_r, gc_i, rs_r, rs_i, rc_r, rc_i;
 };
 
-__global__ void __launch_bounds__(NT) accumulate_partial_kernel(int nslot, int M, int N, int b, const zc *Wt,
-                                                                long long nomega, long long w0, const zc *G,
-                                                                const zc *R, long long ldX, const zc *scal,
-                                                                int ngroups, AccPart *part, AccPart *part_hs,
-                                                                int conj_w) {
+__global__ void __launch_bounds__(ACC_NT) accumulate_partial_kernel(int nslot, int M, int N, int b, const zc *Wt,
+                                                                    long long nomega, long long w0,
+                                                                    const zc *__restrict__ G, const zc *__restrict__ R,
+                                                                    long long ldX, const zc *det, const zc *e1,
+                                                                    const zc *e2, AccPart *part, int conj_w) {
+    __shared__ zc s_c[ACC_GROUP], s_h[ACC_GROUP];
     const long long MN = (long long)M * N;
-    const long long nel = (long long)nslot * MN;
-    const long long total = nel * ngroups;
-    for (long long t = blockIdx.x * (long long)NT + threadIdx.x; t < total; t += (long long)gridDim.x * NT) {
-        const int q = (int)(t / nel);
-        const long long e = t - (long long)q * nel;
-        const int s = (int)(e / MN);
-        const long long rj = e - (long long)s * MN;
-        const long long r = rj / N, j = rj - r * N;
-        const int wa = q * ACC_GROUP, wb = min(b, wa + ACC_GROUP);
-        const zc *wrow = Wt + (long long)s * nomega + w0;
+    const long long e = blockIdx.x * (long long)ACC_NT + threadIdx.x;
+    const int q = blockIdx.y, wa = q * ACC_GROUP, nw = min(b - wa, ACC_GROUP);
+    const long long r = e / N, j = e - r * N;
+    const zc *g = G + r * ldX + (long long)wa * N + j, *x = R + r * ldX + (long long)wa * N + j;
+    for (int s = blockIdx.z; s < nslot; s += gridDim.z) {
+        __syncthreads();
+        if (threadIdx.x < nw) {
+            const int w = wa + threadIdx.x;
+            const zc c = Wt[(long long)s * nomega + w0 + w] * det[w];
+            s_c[threadIdx.x] = conj_w ? conjz(c) : c;
+            s_h[threadIdx.x] = e1 ? e1[w] + e2[w] : mkz(0.0, 0.0);
+        }
+        __syncthreads();
+        if (e > MN) continue;
         AccPart P = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int w = wa; w < wb; ++w) {
-            const zc wt = conj_w ? conjz(wrow[w]) : wrow[w];
-            const long long o = r * ldX + (long long)w * N + j;
-            const zc tg = wt * G[o], tr = wt * R[o];
-            neumaier(P.gs_r, P.gc_r, tg.x);
-            neumaier(P.gs_i, P.gc_i, tg.y);
-            neumaier(P.rs_r, P.rc_r, tr.x);
-            neumaier(P.rs_i, P.rc_i, tr.y);
-        }
-        part[t] = P;
-        if (rj == 0 && scal) {  // the two scalars of the slot ride on the element (s, 0, 0)
-            AccPart Q = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int w = wa; w < wb; ++w) {
-                const zc wt = conj_w ? conjz(wrow[w]) : wrow[w];
-                const zc th = wt * scal[2 * w], ts = wt * scal[2 * w + 1];
-                neumaier(Q.gs_r, Q.gc_r, th.x);
-                neumaier(Q.gs_i, Q.gc_i, th.y);
-                neumaier(Q.rs_r, Q.rc_r, ts.x);
-                neumaier(Q.rs_i, Q.rc_i, ts.y);
+        for (int w4 = 0; w4 < nw; w4 += 4) {
+            zc gv[4], xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                gv[u] = mkz(0.0, 0.0);
+                xv[u] = mkz(1.0, 0.0);  // element MN: c h and c
+                if (e < MN && w4 + u < nw) {
+                    gv[u] = g[(long long)(w4 + u) * N];
+                    xv[u] = x[(long long)(w4 + u) * N];
+                }
             }
-            part_hs[(long long)q * nslot + s] = Q;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (w4 + u < nw) {
+                    const zc c = s_c[w4 + u];
+                    const zc tg = c * (e1 ? gv[u] + s_h[w4 + u] * xv[u] : gv[u]), tr = c * xv[u];
+                    neumaier(P.gs_r, P.gc_r, tg.x);
+                    neumaier(P.gs_i, P.gc_i, tg.y);
+                    neumaier(P.rs_r, P.rc_r, tr.x);
+                    neumaier(P.rs_i, P.rc_i, tr.y);
+                }
         }
+        part[((long long)q * nslot + s) * (MN + 1) + e] = P;
     }
 }
 
@@ -172,18 +168,22 @@ __device__ __forceinline__ void add_part(double &s, double &c, double ps, double
     c += pc;
 }
 
-__global__ void __launch_bounds__(NT) accumulate_final_kernel(int nslot, int M, int N, const int *slotmap,
-                                                              int ngroups, const AccPart *part,
-                                                              const AccPart *part_hs, zc *accG, zc *compG, zc *accR,
-                                                              zc *compR, zc *accHS, zc *compHS) {
-    const long long MN = (long long)M * N;
-    const long long nel = (long long)nslot * MN;
-    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < nel; e += (long long)gridDim.x * NT) {
-        const int s = (int)(e / MN);
-        const long long rj = e - (long long)s * MN;
-        const long long a = (long long)slotmap[s] * MN + rj;
-        double gs_r = accG[a].x, gs_i = accG[a].y, gc_r = compG[a].x, gc_i = compG[a].y;
-        double rs_r = accR[a].x, rs_i = accR[a].y, rc_r = compR[a].x, rc_i = compR[a].y;
+__global__ void __launch_bounds__(ACC_NT) accumulate_final_kernel(int nslot, int M, int N, const int *slotmap,
+                                                                  int ngroups, const AccPart *__restrict__ part,
+                                                                  zc *accG, zc *compG, zc *accR, zc *compR, zc *accHS,
+                                                                  zc *compHS) {
+    const long long MN = (long long)M * N, nel = (long long)nslot * (MN + 1);
+    for (long long e = blockIdx.x * (long long)ACC_NT + threadIdx.x; e < nel; e += (long long)gridDim.x * ACC_NT) {
+        const int s = (int)(e / (MN + 1));
+        const long long rj = e - (long long)s * (MN + 1);
+        const bool scalars = rj == MN;
+        if (scalars && !accHS) continue;
+        const long long a = scalars ? 2LL * slotmap[s] : (long long)slotmap[s] * MN + rj;
+        zc *pg = scalars ? accHS : accG, *pgc = scalars ? compHS : compG;
+        zc *pr = scalars ? accHS + 1 : accR, *prc = scalars ? compHS + 1 : compR;
+        double gs_r = pg[a].x, gs_i = pg[a].y, gc_r = pgc[a].x, gc_i = pgc[a].y;
+        double rs_r = pr[a].x, rs_i = pr[a].y, rc_r = prc[a].x, rc_i = prc[a].y;
+#pragma unroll 4
         for (int q = 0; q < ngroups; ++q) {
             const AccPart P = part[(long long)q * nel + e];
             add_part(gs_r, gc_r, P.gs_r, P.gc_r);
@@ -191,33 +191,45 @@ __global__ void __launch_bounds__(NT) accumulate_final_kernel(int nslot, int M, 
             add_part(rs_r, rc_r, P.rs_r, P.rc_r);
             add_part(rs_i, rc_i, P.rs_i, P.rc_i);
         }
-        accG[a] = mkz(gs_r, gs_i);
-        compG[a] = mkz(gc_r, gc_i);
-        accR[a] = mkz(rs_r, rs_i);
-        compR[a] = mkz(rc_r, rc_i);
-        if (rj == 0 && accHS) {
-            const long long ah = 2LL * slotmap[s];
-            double hs_r = accHS[ah].x, hs_i = accHS[ah].y, hc_r = compHS[ah].x, hc_i = compHS[ah].y;
-            double ss_r = accHS[ah + 1].x, ss_i = accHS[ah + 1].y, sc_r = compHS[ah + 1].x, sc_i = compHS[ah + 1].y;
-            for (int q = 0; q < ngroups; ++q) {
-                const AccPart Q = part_hs[(long long)q * nslot + s];
-                add_part(hs_r, hc_r, Q.gs_r, Q.gc_r);
-                add_part(hs_i, hc_i, Q.gs_i, Q.gc_i);
-                add_part(ss_r, sc_r, Q.rs_r, Q.rc_r);
-                add_part(ss_i, sc_i, Q.rs_i, Q.rc_i);
-            }
-            accHS[ah] = mkz(hs_r, hs_i);
-            compHS[ah] = mkz(hc_r, hc_i);
-            accHS[ah + 1] = mkz(ss_r, ss_i);
-            compHS[ah + 1] = mkz(sc_r, sc_i);
-        }
+        pg[a] = mkz(gs_r, gs_i);
+        pgc[a] = mkz(gc_r, gc_i);
+        pr[a] = mkz(rs_r, rs_i);
+        prc[a] = mkz(rc_r, rc_i);
     }
 }
 
-// a[i] += c[i]  (fold the compensation terms into the sums)
-__global__ void fold_comp_kernel(long long n, zc *a, const zc *c) {
-    for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < n; i += (long long)gridDim.x * NT)
-        a[i] = a[i] + c[i];
+// out[i] = v through two 8-byte stores: the caller's buffers are aligned to a double only
+__device__ __forceinline__ void store8(zc *out, long long i, zc v) {
+    double *d = reinterpret_cast<double *>(out) + 2 * i;
+    d[0] = v.x;
+    d[1] = v.y;
+}
+
+// The accumulated sums with their compensations: out[slot][r] = acc[slot][src(r)] + comp[slot][src(r)], averaged with
+// the ket side's sums where given; src(r) = rowmap[r] (null: r).  Block rows 0 .. 2 nslot - 1 are the gradient and
+// density matrices, one more holds the scalars.
+__global__ void fold_out_kernel(int nslot, int M, int N, const int *rowmap, FoldSums S, zc *outG, zc *outR,
+                                zc *outHS) {
+    const long long MN = (long long)M * N;
+    for (long long y = blockIdx.y; y < 2LL * nslot + 1; y += gridDim.y) {
+        if (y == 2LL * nslot) {
+            for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < 2LL * nslot; i += (long long)gridDim.x * NT)
+                store8(outHS, i, S.HS[i] + S.cHS[i]);
+            continue;
+        }
+        const long long slot = y >> 1;
+        const bool dens = y & 1;
+        const zc *acc = dens ? S.R : S.G, *comp = dens ? S.cR : S.cG;
+        const zc *ka = dens ? S.KR : S.KG, *kc = dens ? S.cKR : S.cKG;
+        zc *out = (dens ? outR : outG) + slot * MN;
+        for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < MN; e += (long long)gridDim.x * NT) {
+            const long long r = e / N, j = e - r * N;
+            const long long o = slot * MN + (rowmap ? (long long)rowmap[r] * N + j : e);
+            zc v = acc[o] + comp[o];
+            if (ka) v = 0.5 * (v + (ka[o] + kc[o]));
+            store8(out, e, v);
+        }
+    }
 }
 
 // H2r[(i M + k) M^2 + (l M + j)] = H2(i, j, k, l) with H2 in Fortran order (MakeGamma operand
@@ -231,15 +243,12 @@ __global__ void permute_h2_kernel(int M, const zc *H2, zc *H2r) {
     }
 }
 
-// out[r*N + j] = in[rowmap[r]*ldin + j]  (row permutation of an M x N matrix, batched by blockIdx.y)
-__global__ void permute_rows_kernel(int M, int N, const int *rowmap, const zc *in, long long ldin, long long bs_in,
-                                    zc *out, long long bs_out) {
+// out[r] = in[rowmap[r]] (M x N), into two buffers
+__global__ void permute_rows_kernel(int M, int N, const int *rowmap, const zc *in, zc *out, zc *out2) {
     const long long tot = (long long)M * N;
-    const zc *src = in + blockIdx.y * bs_in;
-    zc *dst = out + blockIdx.y * bs_out;
     for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < tot; e += (long long)gridDim.x * NT) {
-        long long r = e / N, j = e - r * N;
-        dst[e] = src[(long long)rowmap[r] * ldin + j];
+        const long long r = e / N, j = e - r * N;
+        out[e] = out2[e] = in[(long long)rowmap[r] * N + j];
     }
 }
 
@@ -326,22 +335,6 @@ __global__ void ket_prep_kernel(int M, int N, int b, const zc *Hb, const zc *bra
         const zc hb = Hb ? Hb[r * N + j] : mkz(0.0, 0.0);
         V[r * ld + c] = V[r * ld + c] + hb + h * bra[r * N + j];
     }
-}
-
-// P_w <- conj(det_w) P_w
-__global__ void scale_conj_det_kernel(int M, int N, int b, const zc *det, zc *P, long long ld) {
-    const long long total = (long long)M * b * N;
-    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < total; e += (long long)gridDim.x * NT) {
-        long long r = e / ((long long)b * N), c = e - r * ((long long)b * N);
-        int w = (int)(c / N);
-        P[r * ld + c] = conjz(det[w]) * P[r * ld + c];
-    }
-}
-
-// out = (a + b) / 2
-__global__ void average_kernel(long long n, const zc *a, const zc *b, zc *out) {
-    for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < n; i += (long long)gridDim.x * NT)
-        out[i] = 0.5 * (a[i] + b[i]);
 }
 
 // Y_w = R1[il] T2[:, rem] for a spin rotation R1 that is block diagonal with one 2 x 2 block per
@@ -527,37 +520,31 @@ int launch_add_inplace(int M, int N, int b, const zc *A, zc *G, long long ldX, c
     return PHF_OK;
 }
 
-int launch_epilogue(int M, int N, int b, zc *G, zc *X, long long ldX, const zc *det, const zc *e1,
-                    const zc *e2, zc *scal, cudaStream_t st) {
-    ProfScope prof(st, PROF_MEMORY);
-    epilogue_kernel<<<grid_for((long long)M * b * N), NT, 0, st>>>(M, N, b, G, X, ldX, det, e1, e2, scal);
-    ++g_launches;
-    PHF_CHECK_LAUNCH();
-    return PHF_OK;
-}
-
 size_t accumulate_scratch_bytes(int nslot, int M, int N, int b) {
     const long long ngroups = (b + ACC_GROUP - 1) / ACC_GROUP;
     return (size_t)ngroups * ((size_t)nslot * M * N + nslot) * sizeof(AccPart);
 }
 
 int launch_accumulate(int nslot, int M, int N, int b, const zc *Wt, long long nomega, long long w0, const int *slotmap,
-                      const zc *G, const zc *R, long long ldX, const zc *scal, zc *accG, zc *compG, zc *accR,
-                      zc *compR, zc *accHS, zc *compHS, void *scratch, cudaStream_t st, int conj_weights) {
+                      const zc *G, const zc *R, long long ldX, const zc *det, const zc *e1, const zc *e2, zc *accG,
+                      zc *compG, zc *accR, zc *compR, zc *accHS, zc *compHS, void *scratch, cudaStream_t st,
+                      int conj_weights) {
     const int ngroups = (b + ACC_GROUP - 1) / ACC_GROUP;
     AccPart *part = reinterpret_cast<AccPart *>(scratch);
-    AccPart *part_hs = part + (size_t)ngroups * nslot * M * N;
+    const long long nel = (long long)M * N + 1;
     {
         ProfScope prof(st, PROF_MEMORY);
-        accumulate_partial_kernel<<<grid_for((long long)ngroups * nslot * M * N), NT, 0, st>>>(
-            nslot, M, N, b, Wt, nomega, w0, G, R, ldX, scal, ngroups, part, part_hs, conj_weights);
+        const dim3 grid((unsigned)((nel + ACC_NT - 1) / ACC_NT), (unsigned)ngroups, (unsigned)std::min(nslot, 65535));
+        accumulate_partial_kernel<<<grid, ACC_NT, 0, st>>>(nslot, M, N, b, Wt, nomega, w0, G, R, ldX, det, e1, e2, part,
+                                                           conj_weights);
     }
     ++g_launches;
     PHF_CHECK_LAUNCH();
     {
         ProfScope prof(st, PROF_MEMORY);
-        accumulate_final_kernel<<<grid_for((long long)nslot * M * N), NT, 0, st>>>(
-            nslot, M, N, slotmap, ngroups, part, part_hs, accG, compG, accR, compR, accHS, compHS);
+        const long long ctas = std::min<long long>((nslot * nel + ACC_NT - 1) / ACC_NT, 1 << 20);
+        accumulate_final_kernel<<<(unsigned)ctas, ACC_NT, 0, st>>>(nslot, M, N, slotmap, ngroups, part, accG, compG, accR,
+                                                                   compR, accHS, compHS);
     }
     ++g_launches;
     PHF_CHECK_LAUNCH();
@@ -573,25 +560,11 @@ int launch_ket_prep(int M, int N, int b, const zc *Hb, const zc *bra, const zc *
     return PHF_OK;
 }
 
-int launch_scale_conj_det(int M, int N, int b, const zc *det, zc *P, long long ld, cudaStream_t st) {
+int launch_fold_out(int nslot, int M, int N, const int *rowmap, const FoldSums &S, zc *outG, zc *outR, zc *outHS,
+                    cudaStream_t st) {
     ProfScope prof(st, PROF_MEMORY);
-    scale_conj_det_kernel<<<grid_for((long long)M * b * N), NT, 0, st>>>(M, N, b, det, P, ld);
-    ++g_launches;
-    PHF_CHECK_LAUNCH();
-    return PHF_OK;
-}
-
-int launch_average(long long n, const zc *a, const zc *b, zc *out, cudaStream_t st) {
-    ProfScope prof(st, PROF_MEMORY);
-    average_kernel<<<grid_for(n), NT, 0, st>>>(n, a, b, out);
-    ++g_launches;
-    PHF_CHECK_LAUNCH();
-    return PHF_OK;
-}
-
-int launch_fold_comp(long long n, zc *a, const zc *c, cudaStream_t st) {
-    ProfScope prof(st, PROF_MEMORY);
-    fold_comp_kernel<<<grid_for(n), NT, 0, st>>>(n, a, c);
+    fold_out_kernel<<<dim3(grid_for((long long)M * N), (unsigned)std::min(2 * nslot + 1, 65535)), NT, 0, st>>>(
+        nslot, M, N, rowmap, S, outG, outR, outHS);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     return PHF_OK;
@@ -606,11 +579,9 @@ int launch_permute_h2(int M, const zc *H2, zc *H2r, cudaStream_t st) {
     return PHF_OK;
 }
 
-int launch_permute_rows(int M, int N, int nbatch, const int *rowmap, const zc *in, long long ldin, long long bs_in,
-                        zc *out, long long bs_out, cudaStream_t st) {
+int launch_permute_rows(int M, int N, const int *rowmap, const zc *in, zc *out, zc *out2, cudaStream_t st) {
     ProfScope prof(st, PROF_MEMORY);
-    permute_rows_kernel<<<dim3(grid_for((long long)M * N), nbatch), NT, 0, st>>>(M, N, rowmap, in, ldin, bs_in, out,
-                                                                                 bs_out);
+    permute_rows_kernel<<<grid_for((long long)M * N), NT, 0, st>>>(M, N, rowmap, in, out, out2);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     return PHF_OK;
