@@ -14,7 +14,8 @@
 // in isolation): each warp owns a 32 x 16 block of the tile as 4 x 2 blocks of 8 x 8, and a complex product
 // is four real MMAs (re re, -im im, re im, im re), two for a real A.  Bound: the FP64 tensor pipe for long k
 // (real 2080 x 2080 by complex 2080 x 3200: 2.19 -> 1.80 ms, 30.8 TFLOP/s, when the address arithmetic left
-// the k loop), latency for the small products (n = 20, 112 points: GEMMs 230 -> 145 us of an evaluation).
+// the k loop), latency for the small products (n = 20, 112 points: GEMMs 230 -> 145 us of an evaluation, and 87 with
+// the sums of small grids in groups).
 #include <type_traits>
 
 #include "phf_internal.h"
@@ -65,7 +66,7 @@ template <int BM, int BN>
 __host__ __device__ constexpr int zg_stages() { return (BM == BN || BN == 112) ? 3 : 2; }
 
 template <bool AREAL, int BM, int BN>
-constexpr size_t zg_smem_bytes() {
+__host__ __device__ constexpr size_t zg_smem_bytes() {
     return (size_t)zg_stages<BM, BN>() * BK *
            (zg_pitch_a<AREAL>(BM) * (AREAL ? sizeof(double) : sizeof(zc)) + zg_pitch_b(BN) * sizeof(zc));
 }
@@ -77,8 +78,12 @@ constexpr size_t zg_smem_bytes() {
 // complex element, 8 a real one; out-of-range elements are zero-filled) through zg_stages stages;
 // conjugation is applied when fragments are read.  A real B (only the exchange-matrix build) is
 // loaded with plain loads into the same stages.
-template <bool AREAL, int BM, int BN>
-__global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
+//
+// KS > 1: KS groups of such threads, each with its own stages, take consecutive ranges of k-tiles, and the groups'
+// accumulators are added through shared memory in the groups' order.  For grids that leave the chip idle, where a
+// tile's k loop is a chain of load and multiply latencies on one or two of the multiprocessor's four schedulers.
+template <bool AREAL, int BM, int BN, int KS = 1>
+__global__ void __launch_bounds__(KS *zg_threads<BM, BN>(), KS == 1 ? zg_min_blocks<BM, BN>() : 1)
     zgemm_kernel(int m, int n, int k, int nb0, int ntn, zc alpha, View A, View B, zc beta, OutView C,
                  const long long *__restrict__ offs) {
     using TA = typename ATile<AREAL>::T;
@@ -90,10 +95,12 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     constexpr int PA = zg_pitch_a<AREAL>(BM), PB = zg_pitch_b(BN);
     constexpr int ZG_STAGES = zg_stages<BM, BN>();
     extern __shared__ __align__(16) unsigned char zg_smem[];
-    TA *As = reinterpret_cast<TA *>(zg_smem);                                      // [stage][kk][i]
-    zc *Bs = reinterpret_cast<zc *>(zg_smem + (size_t)ZG_STAGES * BK * PA * sizeof(TA));  // [stage][kk][j]
+    const int group = KS == 1 ? 0 : (int)threadIdx.x / NT;
+    unsigned char *stages = zg_smem + (KS == 1 ? 0 : group * zg_smem_bytes<AREAL, BM, BN>());
+    TA *As = reinterpret_cast<TA *>(stages);                                      // [stage][kk][i]
+    zc *Bs = reinterpret_cast<zc *>(stages + (size_t)ZG_STAGES * BK * PA * sizeof(TA));  // [stage][kk][j]
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x - group * NT, lane = tid & 31, warp = tid >> 5;
     const int wr = (warp / WARPS_N) * 32, wc = (warp % WARPS_N) * 16;  // warp block within the tile
     const int fr = lane >> 2, fk = lane & 3;                            // fragment row / k of this lane
     const long long bz = blockIdx.x / ntn;
@@ -108,7 +115,8 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     }
     const bool a_mfast = (A.rs == 1);  // element order of the A tile loads
     const bool b_nfast = (B.cs == 1);
-    const int nkt = (k + BK - 1) / BK;
+    const int nkt_all = (k + BK - 1) / BK;
+    const int per = (nkt_all + KS - 1) / KS, kt0 = group * per, nkt = max(0, min(per, nkt_all - kt0));
     // Each thread's r-th element of a tile is dA rows (or k's) and a fixed pointer and shared-memory step after
     // its first; the pointers advance by one k-tile per load_stage call (addresses from scratch for every
     // element were three of five instructions of the k loop).
@@ -118,9 +126,10 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     const int bj = b_nfast ? tid % BN : tid / BK, bk = b_nfast ? tid / BN : tid % BK;
     const int bsz = B.real ? (int)sizeof(double) : (int)sizeof(zc);
     const unsigned char *pa = reinterpret_cast<const unsigned char *>(A.p) +
-                              (oa + (long long)(row0 + ai) * A.rs + (long long)ak * A.cs) * (long long)sizeof(TA);
+                              (oa + (long long)(row0 + ai) * A.rs + (long long)(kt0 * BK + ak) * A.cs) *
+                                  (long long)sizeof(TA);
     const unsigned char *pb = reinterpret_cast<const unsigned char *>(B.p) +
-                              (ob + (long long)bk * B.rs + (long long)(col0 + bj) * B.cs) * bsz;
+                              (ob + (long long)(kt0 * BK + bk) * B.rs + (long long)(col0 + bj) * B.cs) * bsz;
     const long long astep = (long long)(a_mfast ? RA * A.cs : KA * A.rs) * (long long)sizeof(TA),
                     bstep = (long long)(b_nfast ? RB * B.rs : KA * B.cs) * bsz;
     const uint32_t sa0 = (uint32_t)__cvta_generic_to_shared(As) + (uint32_t)((ak * PA + ai) * sizeof(TA)),
@@ -136,7 +145,7 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     for (int r = 0; r < LB; ++r)
         if (col0 + bj + (b_nfast ? 0 : KA * r) < n && ((BN * BK) % NT == 0 || tid + NT * r < BN * BK)) bmask |= 1u << r;
 
-    auto load_stage = [&](int stage, int kt) {  // called for kt = 0, 1, 2, ... in turn
+    auto load_stage = [&](int stage, int kt) {  // called for kt = kt0, kt0 + 1, ... in turn
         unsigned am = amask, bm = bmask;
         if ((kt + 1) * BK > k) {  // the last k-tile
             const int ka = k - kt * BK - ak, kb = k - kt * BK - bk;
@@ -186,12 +195,16 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
 
 #pragma unroll
     for (int st = 0; st < ZG_STAGES - 1; ++st) {
-        if (st < nkt) load_stage(st, st);
+        if (st < nkt) load_stage(st, kt0 + st);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int kt = 0; kt < nkt; ++kt) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ZG_STAGES - 2) : "memory");
-        __syncthreads();  // stage kt landed for every thread; stage kt - 1 is no longer read
+        // stage kt landed for every thread of the group; stage kt - 1 is no longer read
+        if constexpr (KS == 1)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(NT) : "memory");
         const int stage = kt % ZG_STAGES;
         const TA *At = As + (size_t)stage * BK * PA;
         const zc *Bt = Bs + (size_t)stage * BK * PB;
@@ -220,7 +233,7 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
                 }
             }
         };
-        const int krem = k - kt * BK;
+        const int krem = k - (kt0 + kt) * BK;
         if (ni == 4 && nj == 2 && krem >= BK) {
 #pragma unroll
             for (int kk = 0; kk < BK; kk += 4) step(kk, std::true_type{});
@@ -229,13 +242,48 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
             for (int kk = 0; kk < min(BK, krem); kk += 4) step(kk, std::false_type{});
         }
         const int kn = kt + ZG_STAGES - 1;  // refill the stage computed in the previous iteration
-        if (kn < nkt) load_stage(kn % ZG_STAGES, kn);
+        if (kn < nkt) load_stage(kn % ZG_STAGES, kt0 + kn);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if constexpr (KS > 1) {
+        // every group's accumulators to shared memory; group g then finishes row blocks g, g + KS, ..
+        static_assert(KS * NT * 32 * sizeof(double) <= KS * zg_smem_bytes<AREAL, BM, BN>(), "reduction buffer");
+        double *red = reinterpret_cast<double *>(zg_smem);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    red[((group * 4 + i) * 8 + j * 4 + h * 2) * NT + tid] = cr[i][j][h];
+                    red[((group * 4 + i) * 8 + j * 4 + h * 2 + 1) * NT + tid] = ci[i][j][h];
+                }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i % KS != group) continue;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double *p = red + (i * 8 + j * 4 + h * 2) * NT + tid;
+                    double x = p[0], y = p[NT];
+#pragma unroll
+                    for (int g = 1; g < KS; ++g) {
+                        x += p[g * 32 * NT];
+                        y += p[g * 32 * NT + NT];
+                    }
+                    cr[i][j][h] = x;
+                    ci[i][j][h] = y;
+                }
+        }
+    }
     const bool use_beta = (beta.x != 0.0 || beta.y != 0.0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+        if (KS > 1 && i % KS != group) continue;
         const int gi = row0 + wr + 8 * i + fr;
         if (gi >= m) continue;
 #pragma unroll
@@ -268,7 +316,7 @@ __global__ void __launch_bounds__(zg_threads<BM, BN>(), zg_min_blocks<BM, BN>())
     }
 }
 
-template <int BM, int BN>
+template <int BM, int BN, int KS = 1>
 int launch_tile(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, const View &B, zc beta,
                 const OutView &C, const long long *offs, cudaStream_t st) {
     const int ntn = (n + BN - 1) / BN, ntm = (m + BM - 1) / BM;
@@ -280,19 +328,19 @@ int launch_tile(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, 
     }
     dim3 grid((unsigned)gx, (unsigned)ntm, 1);
     if (A.real) {
-        constexpr size_t smem = zg_smem_bytes<true, BM, BN>();
-        PHF_CUDA(cudaFuncSetAttribute(zgemm_kernel<true, BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        constexpr size_t smem = KS * zg_smem_bytes<true, BM, BN>();
+        PHF_CUDA(cudaFuncSetAttribute(zgemm_kernel<true, BM, BN, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
         ProfScope prof(st, -1);
-        zgemm_kernel<true, BM, BN><<<grid, zg_threads<BM, BN>(), smem, st>>>(m, n, k, nb0, ntn, alpha, A, B, beta, C,
-                                                                             offs);
+        zgemm_kernel<true, BM, BN, KS><<<grid, KS * zg_threads<BM, BN>(), smem, st>>>(m, n, k, nb0, ntn, alpha, A, B,
+                                                                                      beta, C, offs);
     } else {
-        constexpr size_t smem = zg_smem_bytes<false, BM, BN>();
-        PHF_CUDA(cudaFuncSetAttribute(zgemm_kernel<false, BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        constexpr size_t smem = KS * zg_smem_bytes<false, BM, BN>();
+        PHF_CUDA(cudaFuncSetAttribute(zgemm_kernel<false, BM, BN, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
         ProfScope prof(st, -1);
-        zgemm_kernel<false, BM, BN><<<grid, zg_threads<BM, BN>(), smem, st>>>(m, n, k, nb0, ntn, alpha, A, B, beta,
-                                                                              C, offs);
+        zgemm_kernel<false, BM, BN, KS><<<grid, KS * zg_threads<BM, BN>(), smem, st>>>(m, n, k, nb0, ntn, alpha, A, B,
+                                                                                       beta, C, offs);
     }
     ++g_launches;
     PHF_CHECK_LAUNCH();
@@ -300,7 +348,7 @@ int launch_tile(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, 
 }
 
 // Tile shape 0 = 64 x 64, 1 = 128 x 32, 2 = 32 x 128, 3 = 32 x 112, 4 = 64 x 112, 5 = 32 x 32,
-// 6 = 32 x 64.
+// 6 = 32 x 64; 7 and 8 = 32 x 32 with k in four and two groups.
 int launch_choice(int tile, int m, int n, int k, int nb0, int nb1, zc alpha, const View &A, const View &B, zc beta,
                   const OutView &C, const long long *offs, cudaStream_t st) {
     if (tile == 1) return launch_tile<128, 32>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
@@ -309,6 +357,8 @@ int launch_choice(int tile, int m, int n, int k, int nb0, int nb1, zc alpha, con
     if (tile == 4) return launch_tile<64, 112>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     if (tile == 5) return launch_tile<32, 32>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     if (tile == 6) return launch_tile<32, 64>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
+    if (tile == 7) return launch_tile<32, 32, 4>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
+    if (tile == 8) return launch_tile<32, 32, 2>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     return launch_tile<64, 64>(m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
 }
 
@@ -325,6 +375,15 @@ int zgemm_strided(int m, int n, int k, int nb0, int nb1, zc alpha, const View &A
         set_error(PHF_ERR_ARG, "zgemm_strided: k <= 0");
         return PHF_ERR_ARG;
     }
+    // Few 32 x 32 tiles over a long sum: the sum in groups of a block.  A tile's two warps use two of the four
+    // schedulers and wait for every k-tile, so up to one block a multiprocessor takes four groups (16 tiles over k =
+    // 400: 19.7 -> 10.3 us; 98 over 210: 20.1 -> 11.1; 35 over 40: 9.4 -> 6.8), up to two take two (195 over 96: 16.6
+    // -> 14.5), and long sums take four groups up to three (200 over 1600: 175 -> 144 us, 325 real ones over 2080:
+    // 173 -> 142; from four blocks a multiprocessor on, all schedulers are busy without).  The groups add in another
+    // order than the other tiles, so such a shape has no other candidates.
+    const long long tiles = (long long)nb0 * nb1 * ((m + 31) / 32) * ((n + 31) / 32);
+    if (k > 2 * BK && tiles <= (k >= 16 * BK ? 444 : 296))
+        return launch_choice(tiles <= 148 || k >= 16 * BK ? 7 : 8, m, n, k, nb0, nb1, alpha, A, B, beta, C, offs, st);
     const TuneKey key{0, (long long)m, (long long)n, (long long)k, (long long)nb0 * 65536 + nb1,
                       (long long)(A.real * 4 + B.real * 2 + C.real) * 2 + (offs != nullptr)};
     if (t_tune_record)
