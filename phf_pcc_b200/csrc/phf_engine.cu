@@ -44,6 +44,14 @@ unsigned long long g_launches = 0;
 int g_narrow_mma = 0;
 int g_fx_i8 = 1;
 
+// Whether a tensor-core plan forms its densities (and F X) by int8 slice products: n > 64 with up to seven slices, but
+// in the residue form from n > 128 only.  Up to there the FP64 products are the faster ones, without slicing passes
+// over X, the densities and Gamma: an evaluation at n = 72 (112 points) takes 0.62 against 0.68 ms, n = 101 (156
+// points) 1.53 against 1.61, n = 128 (800 points) 11.8 against 12.2; n = 150 (156 points) 11.46 against 11.34.
+static bool density_i8(const PlanImpl &p) {
+    return !oz_rho_slice_ok(p.n) && p.slices <= 7 && !(p.rz && p.n <= 128);
+}
+
 // ---------------------------------------------------------------- per-class event timing
 namespace {
 struct ProfState {
@@ -694,7 +702,8 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
             else per += (8 * (n2 + 64) * oz_slots(p.slices)) / sizeof(zc) + 1  // exchange slices
                         + (2 * n2 + 2 * (size_t)p.L) * oz_slots(p.slices) / sizeof(zc) + 1    // Coulomb slices
                         + p.L + n2;                                                // d^T, J pairs
-            // int8 density GEMM: the X rows' slices and exponents
+            // int8 density GEMM: the X rows' slices and exponents (counted for n <= 128 too, where the residue form
+            // does without: a given workspace makes the same chunks)
             if (p.prec != PHF_PREC_FP64 && !oz_rho_slice_ok(n) && p.slices <= 7) {
                 per += ((size_t)M * oz_pad_k(2LL * N) * oz_slots(p.slices) + 4 * (size_t)M) / sizeof(zc) + 1;
                 // F X on the int8 path: the slices and exponents of X's columns and F's rows
@@ -794,8 +803,8 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
                 PHF_TRY(p.arena.alloc(&p.dpart, (size_t)kDSplit * 2 * b * (size_t)p.L));
                 PHF_TRY(p.arena.alloc(&p.Jr, 2 * b * n2));
             }
-            // n > 64 with int8 slices: rho_w = X_w bra^H for the whole chunk as one int8 GEMM
-            p.rho_i8 = !oz_rho_slice_ok(n) && p.slices <= 7;
+            // rho_w = X_w bra^H for the whole chunk as one int8 GEMM
+            p.rho_i8 = density_i8(p);
             if (p.rho_i8) {
                 const long long xrows = oz_pad_rows((long long)M * p.b), brows = oz_pad_cols(2LL * M);
                 PHF_TRY(p.arena.alloc(&p.Xsl, oz_slice_bytes(xrows, 2LL * N, p.slices)));
@@ -1216,7 +1225,7 @@ int gamma_x_eri(PlanImpl &p, int bc, cudaStream_t st) {
     const long long ld = (long long)b * N, MM = (long long)M * M, n2 = (long long)n * n;
     // tensor-core path with n <= 64: the operand columns are formed and sliced in one kernel, no density in HBM
     const bool fused = p.prec != PHF_PREC_FP64 && oz_rho_slice_ok(n) && !p.rz;
-    // n > 64 with int8 slices: the densities of the whole chunk as ONE int8 GEMM.  Row (w, i) of X,
+    // rho_i8: the densities of the whole chunk as ONE int8 GEMM.  Row (w, i) of X,
     // X_w[i][:] at Xs + (i b + w) N, is a row of 2N reals (re, im interleaved), and rho_w[i][j] =
     // sum_k X_w[i][k] conj(bra[j][k]) is its product with rows 2j (real part) and 2j + 1 (imaginary
     // part) of the bra's 2M x 2N operand: the (M bc) x 2M reals are the points' densities one after
