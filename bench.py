@@ -213,13 +213,23 @@ def jk_form_of(p):
     return "eri" if p.n <= 128 else "streamed"
 
 
-def sym_active(p, form, precision, sym="auto"):
+RESIDUES = 11  # moduli of the default int8 form
+
+
+def residue_form(p, form, precision, slices, sym="auto"):
+    """Whether the library runs J and K as products of residues modulo eleven moduli: the int8 form with the
+    default `slices` (0) wherever it runs the exchange symmetry."""
+    return precision == "ozaki_i8" and slices == 0 and sym != "off" and (form == "eri" or p.n > 64)
+
+
+def sym_active(p, form, precision, sym="auto", slices=0):
     """Whether the library runs the exchange-matrix form with the exchange symmetry (pairs i <= k against
-    the symmetric half of each density, i < k against the antisymmetric half): on by default in FP64 and,
-    for n > 64, in the tensor-core precisions (the stored form: int8 only)."""
+    the symmetric half of each density, i < k against the antisymmetric half): on by default in FP64, in the
+    residue form and, for n > 64, in the tensor-core precisions (the stored form: int8 only)."""
     if form == "eri" and precision not in ("fp64", "ozaki_i8"):
         return False
-    return form in ("eri", "streamed") and sym != "off" and (precision == "fp64" or p.n > 64)
+    return form in ("eri", "streamed") and sym != "off" and (
+        precision == "fp64" or p.n > 64 or residue_form(p, form, precision, slices, sym))
 
 
 def choose_ipanel(n):
@@ -283,22 +293,33 @@ def jk_regen_flops(p, form, chunks, sym=False, ipanel=0):
 
 
 def tc_reps(precision, slices):
-    """Tensor-core products per FP64-equivalent product: S(S+1)/2 int8 slice products, three BF16
-    products for bf16x3, one TF32 product for tf32."""
+    """Tensor-core products per FP64-equivalent product: S(S+1)/2 int8 slice products (S = 5 for the products
+    that the default form leaves in slices), three BF16 products for bf16x3, one TF32 product for tf32."""
     if precision == "ozaki_i8":
-        return slices * (slices + 1) / 2
+        s = slices or 5
+        return s * (s + 1) / 2
     return 3.0 if precision == "bf16x3" else 1.0
+
+
+def tc_ops_per_point(p, precision, slices, form="eri", sym=True):
+    """Executed tensor-core operations of J and K per grid point (2 per multiply-add).  Residue form: both
+    exchange parities over the p_le = n (n+1)/2 pairs, d and J over them too, eleven products each."""
+    if sym and residue_form(p, form, precision, slices):
+        ple = p.n * (p.n + 1) / 2
+        return RESIDUES * (32.0 * ple * ple + 8.0 * p.L * ple)
+    return tc_reps(precision, slices) * jk_flops_per_point(p, form, sym, precision)
 
 
 def tc_ops_per_step(p, precision, slices, form, chunks, sym=False, ipanel=0):
     """Executed tensor-core operations of the J/K contraction per evaluation (2 per multiply-add)."""
-    return tc_reps(precision, slices) * (jk_flops_per_point(p, form, sym, precision) * p.grid.npoints +
-                                         jk_regen_flops(p, form, chunks, sym, ipanel))
+    return (tc_ops_per_point(p, precision, slices, form, sym) * p.grid.npoints +
+            tc_reps(precision, slices) * jk_regen_flops(p, form, chunks, sym, ipanel))
 
 
-def tc_ops_per_point(p, precision, slices):
-    """Executed tensor-core operations per grid point of the stored-exchange-matrix contractions."""
-    return tc_reps(precision, slices) * (16.0 * p.n ** 4 + 8.0 * p.L * p.n ** 2)
+def int8_dtype(p, form, slices, sym="auto"):
+    if residue_form(p, form, "ozaki_i8", slices, sym):
+        return f"int8 x{RESIDUES} residues (FP64-accurate emulation) + f64"
+    return f"int8 x{slices or 5} slices (FP64-accurate emulation) + f64"
 
 
 def quoted_flops_per_point(p):
@@ -306,23 +327,6 @@ def quoted_flops_per_point(p):
     16 M^2 N + 16 M N^2 + 8 N^3 + 16 M^3 (small algebra)."""
     n, N, M, L = p.n, p.N, p.M, p.L
     return 32.0 * L * n ** 3 + 8.0 * L * n ** 2 + 16.0 * M * M * N + 16.0 * M * N * N + 8.0 * N ** 3 + 16.0 * M ** 3
-
-
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant exchange launch, from
-# ncu captures of these workloads, with the note that says what was captured.
-TRAFFIC = {
-    ("c2", "ozaki_i8"): (2.412e9 + 0.820e9,
-                         "DRAM read + write of the K launch (4096 x 25600 x 4096, the whole 3200-point chunk, wide "
-                         "MMA issue) from an ncu capture of this workload; algorithmic bytes of that "
-                         "launch: A slices 84 MB + B slices 524 MB + FP64 output 839 MB = 1.45e9"),
-    ("c5", "ozaki_i8"): (39.0e9,
-                         "DRAM read + write of the first panel's symmetric exchange GEMM (7059 pair rows x 25600 x "
-                         "20100, the exchange symmetry's largest launch), scaled by the columns (points) from an ncu "
-                         "capture of the same panel on a 384-point grid (4.68 GB for 7059 x 3072 x 20100; an upper "
-                         "estimate, the A-slice reads do not grow with the columns); algorithmic bytes of the full "
-                         "launch: A slices 0.71 GB + B slices 2.58 GB + FP64 output at both mirror positions "
-                         "2.89 GB = 6.2e9"),
-}
 
 
 def measure_int8_peak(torch, dev):
@@ -560,11 +564,11 @@ def run_ours(args):
     C = torch.from_numpy(p.C).to(dev)
     stream = torch.cuda.current_stream(dev)
     flush = torch.empty(int(256e6) // 4, dtype=torch.float32, device=dev)  # > L2 (126 MB)
-    slices = args.slices or 5
+    slices = args.slices
 
     tune = not args.no_autotune
     xs = {"auto": "auto", "on": True, "off": False}[args.exchange_symmetry]
-    sym = sym_active(p, form, args.precision, args.exchange_symmetry)
+    sym = sym_active(p, form, args.precision, args.exchange_symmetry, slices)
     plan = api.Plan(ref=np.eye(p.M), h=p.h, B=p.B, precision=args.precision, slices=args.slices, jk_form=form,
                     autotune=tune, exchange_panel=args.exchange_panel, exchange_symmetry=xs, **kw)
     clk = clock_sampler(local)
@@ -676,7 +680,7 @@ def run_ours(args):
         for prec, r in study.items():
             r["meets_1e-8_Eh"] = r["abs_dE_vs_fp64"] <= 1e-8
             r["meets_1e-7_grad"] = r["max_abs_dgrad_vs_fp64"] <= 1e-7
-            r["tc_tops"] = tc_ops_per_step(p, prec, slices, form, chunks, sym_active(p, form, prec, args.exchange_symmetry),
+            r["tc_tops"] = tc_ops_per_step(p, prec, slices, form, chunks, sym_active(p, form, prec, args.exchange_symmetry, slices),
                                            args.exchange_panel) / (r["jk_ms_per_step"] * 1e-3) / 1e12
 
     e2e_val = statistics.median(e2e_vals) * world if e2e_vals else None
@@ -704,11 +708,9 @@ def run_ours(args):
             achieved = (tc_ops_per_step(p, args.precision, slices, form, chunks, sym, args.exchange_panel) * args.steps
                         / (jk_ms * 1e-3) / 1e12)
             unit = {"ozaki_i8": "TOP/s (int8)", "bf16x3": "TFLOP/s (bf16)", "tf32": "TFLOP/s (tf32)"}[args.precision]
-            traffic = TRAFFIC.get((args.config, args.precision))
             roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": unit,
                     "frac": achieved / peak if peak else None,
-                    "traffic": traffic[0] if traffic else None,
-                    "traffic_note": traffic[1] if traffic else "no ncu capture of this workload's exchange launch",
+                    "traffic": None, "traffic_note": "no ncu capture of this workload's exchange launch",
                     "peak_source": (_peak_source(peaks, {"ozaki_i8": "2 x (dense int8 rate = 2 x bf16 on B200)",
                                                          "bf16x3": "1 x", "tf32": "0.5 x (dense TF32 rate)"}
                                                  [args.precision])
@@ -716,8 +718,11 @@ def run_ours(args):
                     "int8_cublaslt_tops_measured": i8,
                     "frac_of_cublaslt_int8": achieved / i8 if i8 else None,
                     "bf16_tflops_measured": bf16,
-                    "kernel": "ozaki_i8_gemm_kernel (tcgen05 kind::%s, exchange, exchange-row regeneration and "
-                              "Coulomb GEMMs)" % {"ozaki_i8": "i8", "bf16x3": "f16 (bf16)", "tf32": "tf32"}[args.precision],
+                    "kernel": ("residue_gemm_kernel (tcgen05 kind::i8, exchange and Coulomb GEMMs) and "
+                               "ozaki_i8_gemm_kernel (exchange-row regeneration, densities)"
+                               if residue_form(p, form, args.precision, slices, args.exchange_symmetry) else
+                               "ozaki_i8_gemm_kernel (tcgen05 kind::%s, exchange, exchange-row regeneration and Coulomb "
+                               "GEMMs)" % {"ozaki_i8": "i8", "bf16x3": "f16 (bf16)", "tf32": "tf32"}[args.precision]),
                     "fp64_equivalent_tflops": (alg * p.grid.npoints + regen) * args.steps
                                               / (jk_ms * 1e-3) / 1e12,
                     "fp64_dgemm_peak_tflops": fp64_peak}
@@ -744,7 +749,7 @@ def run_ours(args):
             parity = oracle_parity(p, setup[0], block, ora, plist)
             parity["oracle"] = setup[1]
             del setup
-        dtype = {"fp64": "f64", "ozaki_i8": f"int8 x{slices} slices (FP64-accurate emulation) + f64",
+        dtype = {"fp64": "f64", "ozaki_i8": int8_dtype(p, form, slices, args.exchange_symmetry),
                  "bf16x3": "bf16 hi+lo x3 products, f32 accumulation + f64",
                  "tf32": "tf32, f32 accumulation + f64"}[args.precision]
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -907,8 +912,9 @@ def run_batch(args):
     if rank == 0:
         peaks = _peaks()
         jk_ms = prof[0][0]
-        slices = args.slices or 5
-        ops = sum(tc_ops_per_point(p, args.precision, slices) * p.grid.npoints for p in probs)
+        slices = args.slices
+        ops = sum(tc_ops_per_point(p, args.precision, slices, "eri", sym_active(p, "eri", args.precision, "auto", slices))
+                  * p.grid.npoints for p in probs)
         bf16 = peaks.get("bf16_tflops")
         peak = 2.0 * bf16 if bf16 else None
         achieved = ops / (jk_ms * 1e-3) / 1e12 if args.precision != "fp64" else None
@@ -917,7 +923,7 @@ def run_batch(args):
                 "peak_source": _peak_source(peaks, "2 x (dense int8 rate = 2 x bf16 on B200)"),
                 "device_ms_by_class": {k: v[0] for k, v in zip(("jk", "other_gemm", "overlap_inverse", "memory"),
                                                                prof.values())},
-                "kernel": "ozaki_i8_gemm_kernel (all instances' exchange and Coulomb GEMMs)"}
+                "kernel": "residue_gemm_kernel (all instances' exchange and Coulomb GEMMs)"}
         cpu = None
         if not args.no_cpu:
             v, nth, desc, _, _ = cpu_sample(probs[0], seconds_target=args.cpu_seconds)
@@ -927,7 +933,7 @@ def run_batch(args):
         line = {"metric": METRIC, "value": world * pts / (step_ms * 1e-3), "unit": UNIT, "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None,
-                "dtype": "f64" if args.precision == "fp64" else f"int8 x{slices} slices (FP64-accurate emulation) + f64",
+                "dtype": "f64" if args.precision == "fp64" else int8_dtype(probs[0], "eri", slices),
                 "data": "synthetic (seeded h, B_L, determinants per instance)",
                 "config": {"workload": f"{len(probs)} independent instances, n in {sizes}, N = n/2, L = 4n, "
                                        f"grids 112 / 800 points alternating, {pts} points in all",

@@ -55,7 +55,7 @@ enum phf_status {
  * compensated grid sums are FP64 in every mode). */
 enum phf_precision {
     PHF_PREC_FP64 = 0,      /* FP64 CUDA-core GEMMs (the plain FP64 form) */
-    PHF_PREC_OZAKI_I8 = 1,  /* FP64-accurate emulation: int8 slices on tcgen05 tensor cores */
+    PHF_PREC_OZAKI_I8 = 1,  /* FP64-accurate emulation: int8 residues or slices on tcgen05 tensor cores */
     PHF_PREC_BF16X3 = 2,    /* split-BF16 (hi + lo: ~16 significant bits), 3 products, FP32 accumulation (tcgen05) */
     PHF_PREC_TF32 = 3       /* TF32 (11 significant bits), FP32 accumulation (tcgen05) */
 };
@@ -159,7 +159,9 @@ typedef struct {
     const phf_complex *r1, *r2, *rpg;
     const double *weightsp, *weightpg, *roota, *rootb, *rooty;
     int precision;                            /* enum phf_precision */
-    int slices;                               /* int8 slices per operand for PHF_PREC_OZAKI_I8 (0 = default) */
+    int slices;                               /* PHF_PREC_OZAKI_I8: int8 slices per operand, 1..7; 0 = default: J and K
+                                                 from residues modulo eleven 8-bit moduli where the exchange symmetry
+                                                 runs, five slices elsewhere */
     size_t workspace_bytes;                   /* per-chunk workspace budget (0 = default: 6 GiB, or 45 % of
                                                  the free device memory for jk_form 3 when that is more) */
     int jk_form;                              /* Cholesky form only: 0 = automatic, 1 = exchange through the
@@ -324,9 +326,9 @@ int phf_tuned_shapes(void);
    setting.  Plans captured into CUDA graphs keep the form they were captured with. */
 int phf_int8_wide_mma(int on);
 /* Plans created while this is 1 (the default) and that form their densities on the int8 path (int8
-   slices, n > 64; with the default residue products n > 128) also form the per-point product F X = (H1 + J - K) X there: one batched int8 GEMM
-   over the chunk's points (X's columns and F's rows as slices, k = 2M) instead of an FP64 GEMM per
-   point; 0 keeps the FP64 product; a value above 1 also caps the points per sub-batch of that GEMM
+   slices, n > 64; with the default residue products n > 128) also form the per-point product
+   F X = (H1 + J - K) X there: one batched int8 GEMM over the chunk's points (X's columns and F's rows
+   as slices, k = 2M) instead of an FP64 GEMM per point; 0 keeps the FP64 product; a value above 1 also caps the points per sub-batch of that GEMM
    (otherwise sized to 1 GiB of slices).  Returns the previous setting.  No counterpart in the reference. */
 int phf_int8_fock_product(int on);
 /* Library version string. */

@@ -236,7 +236,8 @@ class Plan:
 
     Cholesky form: pass ``h`` (n, n) and ``B`` (L, n, n); dense form: ``hone`` and
     ``htwo``.  Grid arguments as buildhsg.  ``precision`` of the J/K contractions: "fp64",
-    "ozaki_i8" (FP64-accurate int8 tensor-core slices, ``slices`` per operand, default 5),
+    "ozaki_i8" (FP64-accurate int8 tensor-core products: ``slices`` = 0, the default, takes residues modulo
+    eleven moduli where the exchange symmetry runs and five slices elsewhere; 1..7 slices per operand otherwise),
     "bf16x3" (split BF16, three products) or "tf32" (both FP32-accumulated in 512-element segments
     summed in FP64; about 1e-6 relative, far from FP64); ``jk_form``: "auto", "eri"
     (exchange through the n^2 x n^2 spatial ERI matrix, built once and kept), "streamed" (the same

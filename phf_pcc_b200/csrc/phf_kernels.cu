@@ -108,9 +108,10 @@ __device__ __forceinline__ void neumaier(double &s, double &c, double x) {
 //   stage 2: ACC_LANES lanes an element add every ACC_LANES-th group, then each other's sums in a fixed tree, and one
 //            adds the result into the running (acc, comp); a thread for all groups was a chain of 100 loads and
 //            compensated additions for 3200 points (68 against 18 us).
-// Bound: G and R read once; at small sizes the serial chain of the 32 points, so their loads go four ahead (eight: 85 against 75 us at 3200 points) and
-// the group's factors come from shared memory (M = 40 to 96 spin orbitals: 34 us as one load after another, after
-// 4 to 9 us of a separate epilogue that wrote G and R again).
+// Bound: G and R read once; at small sizes the serial chain of the 32 points, so their loads go four ahead (eight
+// take 10 against 11.5 us at M = 40, but 85 against 75 for 3200 points at M = 128) and the group's factors come
+// from shared memory (M = 40 to 96: 12 us against 34 as one load after another, after 4 to 9 us of a separate
+// epilogue that wrote G and R again).
 constexpr int ACC_GROUP = 32, ACC_NT = 128, ACC_LANES = 8;
 
 struct AccPart {
