@@ -2003,7 +2003,8 @@ int plan_eval_batch(PlanImpl *const *plans, int count, const zc *const *d_c, zc 
         bg.h_flags.assign(2 * (size_t)count, 0);
         const int rc = enqueue_batch(plans, count, d_c, d_hs, d_yg, d_yr, bg.branches, bg.d_ptrs, bg.d_flags,
                                      st);
-        if (rc != PHF_OK) {
+        if (rc != PHF_OK) {  // nothing of the batch is left running, whichever branch was not joined
+            for (int b = 0; b < bg.branches; ++b) cudaStreamSynchronize(g_bs.br[b]);
             cudaStreamSynchronize(st);
             cudaGetLastError();
             return rc;
