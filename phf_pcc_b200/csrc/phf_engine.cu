@@ -27,6 +27,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <string>
 #include <vector>
@@ -345,18 +346,36 @@ int choose_ipanel(int n) {
 }  // namespace
 
 namespace {
-// whether every B_L equals its transpose exactly (16 x 16 tiles, so that both sides stay in cache)
-bool cholesky_symmetric(const phf_plan_desc *d) {
+// How the Cholesky vectors compare with their transposes (16 x 16 tiles, so that both sides stay in cache): 2 = every
+// B_L is exactly symmetric, 1 = to rounding, 0 = neither (or not finite).  To rounding: no difference above 2 sqrt(n)
+// units in the last place of the largest element of B_L.  Vectors brought to another basis, X^T B X, are sums of n
+// products on either side and differ by 2 (n = 5), 6 (64), 8 (128) and 10 (200) such units; a difference of that size
+// says nothing about the integrals, and the full rows of vectors that are not symmetric cost twice the exchange work.
+int cholesky_symmetry(const phf_plan_desc *d) {
     const int n = d->nso / 2, T = 16;
+    int level = 2;
     for (int l = 0; l < d->nchol; ++l) {
         const double *B = d->bvec + (size_t)n * n * l;
+        double diff = 0.0;
+        bool exact = true;
         for (int q0 = 0; q0 < n; q0 += T)
             for (int p0 = 0; p0 <= q0; p0 += T)
                 for (int q = q0; q < std::min(q0 + T, n); ++q)
-                    for (int p = p0; p < std::min(p0 + T, q); ++p)
-                        if (B[p + (size_t)n * q] != B[q + (size_t)n * p]) return false;
+                    for (int p = p0; p < std::min(p0 + T, q); ++p) {
+                        const double a = B[p + (size_t)n * q], b = B[q + (size_t)n * p];
+                        if (a != b) {
+                            exact = false;
+                            if (!(std::fabs(a - b) <= std::numeric_limits<double>::max())) return 0;
+                            diff = std::max(diff, std::fabs(a - b));
+                        }
+                    }
+        if (exact) continue;
+        double mx = 0.0;
+        for (size_t e = 0; e < (size_t)n * n; ++e) mx = std::max(mx, std::fabs(B[e]));
+        if (!(diff <= 2.0 * std::sqrt((double)n) * std::numeric_limits<double>::epsilon() * mx)) return 0;
+        level = 1;
     }
-    return true;
+    return level;
 }
 }  // namespace
 
@@ -408,11 +427,13 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
     }
     // the exchange symmetry (n >= 2): the streamed form in FP64 and in the tensor-core forms whose densities
     // are sliced apart from the density GEMM (n > 64); the stored form in FP64 and in the int8 form with
-    // n > 64, when the Cholesky vectors are exactly symmetric (K(rho^T) = K(rho)^T holds for any real
-    // vectors, the Coulomb term over pairs l <= j only for symmetric ones).  The full rows do twice the
+    // n > 64, when the Cholesky vectors are symmetric (K(rho^T) = K(rho)^T holds for any real vectors, the
+    // Coulomb term over pairs l <= j only for symmetric ones; vectors symmetric to rounding are replaced by
+    // (B + B^T) / 2 there).  The full rows do twice the
     // exchange work: an evaluation takes 9.5 ms with them and 5.7 ms without (FP64, n = 64, 800 points),
     // 25.0 and 16.1 ms (int8, n = 128, 800 points), 5.3 and 4.4 ms (int8, n = 101, 312 points)
-    const bool symmetric = p.chol && cholesky_symmetric(d);
+    const int symmetry = p.chol ? cholesky_symmetry(d) : 0;
+    const bool symmetric = symmetry > 0;
     const bool sym_slices = p.prec == PHF_PREC_FP64 || !oz_rho_slice_ok(d->nso / 2);
     if (p.streamed) {
         const int n = d->nso / 2;
@@ -605,17 +626,23 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
     // Hamiltonian
     if (p.chol) {
         const int L = p.L;
-        std::vector<double> hh((size_t)n * n), Bst(symmetric ? 0 : (size_t)L * n * n);
+        // exactly symmetric vectors need no transposition
+        const bool as_given = symmetry == 2, mean = symmetry == 1 && p.ek_sym && !(p.streamed && p.prec == PHF_PREC_FP64);
+        std::vector<double> hh((size_t)n * n), Bst(as_given ? 0 : (size_t)L * n * n);
         for (int i = 0; i < n; ++i)
             for (int j = 0; j < n; ++j) hh[(size_t)i * n + j] = d->h[(size_t)i + (size_t)n * j];
-        for (int l = 0; l < L && !symmetric; ++l)  // (symmetric vectors need no transposition)
+        for (int l = 0; l < L && !as_given; ++l) {
+            const double *B = d->bvec + (size_t)n * n * l;
             for (int pp = 0; pp < n; ++pp)
-                for (int q = 0; q < n; ++q)
-                    Bst[((size_t)l * n + pp) * n + q] = d->bvec[(size_t)pp + (size_t)n * ((size_t)q + (size_t)n * l)];
+                for (int q = 0; q < n; ++q) {
+                    const double a = B[(size_t)pp + (size_t)n * q];
+                    Bst[((size_t)l * n + pp) * n + q] = mean ? 0.5 * a + 0.5 * B[(size_t)q + (size_t)n * pp] : a;
+                }
+        }
         PHF_TRY(p.arena.alloc(&p.h, hh.size()));
         PHF_TRY(p.arena.alloc(&p.Bst, (size_t)L * n * n));
         PHF_CUDA(cudaMemcpy(p.h, hh.data(), hh.size() * sizeof(double), cudaMemcpyHostToDevice));
-        PHF_CUDA(cudaMemcpy(p.Bst, symmetric ? d->bvec : Bst.data(), (size_t)L * n * n * sizeof(double),
+        PHF_CUDA(cudaMemcpy(p.Bst, as_given ? d->bvec : Bst.data(), (size_t)L * n * n * sizeof(double),
                             cudaMemcpyHostToDevice));
         if (p.eri) PHF_TRY(build_exchange_matrix(p));
         // exchange-matrix forms: with h exactly symmetric (H1 = H1^H), H1 is added to Gamma where J is,
