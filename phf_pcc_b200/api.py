@@ -250,9 +250,9 @@ class Plan:
     forms): "auto" (on where available), True or False -- with it the exchange runs over index pairs i <= k
     against the symmetric half of each density and i < k against the antisymmetric half (K(rho^T) =
     K(rho)^T for real integrals): half the exchange GEMM's work.  Streamed form: in FP64 and, for n > 64, in the
-    tensor-core precisions.  Stored form: in FP64 and "ozaki_i8" (with explicit ``slices`` for n > 64), for ``B``
-    symmetric to rounding (2 sqrt(n) ulp of a vector's largest element; (B + B^T) / 2 is taken), full rows
-    otherwise."""
+    tensor-core precisions.  Stored form: in FP64 and "ozaki_i8" (with explicit ``slices`` for n > 64).  All but
+    the streamed FP64 form take it for ``B`` symmetric to rounding (2 sqrt(n) ulp of a vector's largest element;
+    (B + B^T) / 2 is used) and run the full rows otherwise."""
 
     def __init__(self, *, ref, ngrid, nci, cmplxconj, ncisp, nocc, r1, r2, rpg, weightsp, weightpg, roota, rootb,
                  rooty, qj, sp, h=None, B=None, hone=None, htwo=None, precision="fp64", slices=0,

@@ -425,11 +425,11 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
         set_error(PHF_ERR_UNSUPPORTED, "the tensor-core precisions need an exchange-matrix form (jk_form 0, 1 or 3)");
         return PHF_ERR_UNSUPPORTED;
     }
-    // the exchange symmetry (n >= 2): the streamed form in FP64 and in the tensor-core forms whose densities
-    // are sliced apart from the density GEMM (n > 64); the stored form in FP64 and in the int8 form with
-    // n > 64, when the Cholesky vectors are symmetric (K(rho^T) = K(rho)^T holds for any real vectors, the
-    // Coulomb term over pairs l <= j only for symmetric ones; vectors symmetric to rounding are replaced by
-    // (B + B^T) / 2 there).  The full rows do twice the
+    // the exchange symmetry (n >= 2): the streamed form in FP64, and in the tensor-core forms whose densities
+    // are sliced apart from the density GEMM (n > 64); the stored form in FP64 and int8 (residues, and slices with
+    // n > 64).  All but the streamed FP64 form need symmetric Cholesky vectors: K(rho^T) = K(rho)^T holds for any
+    // real vectors, their Coulomb term over pairs l <= j only for symmetric ones (vectors symmetric to rounding are
+    // replaced by (B + B^T) / 2).  The full rows do twice the
     // exchange work: an evaluation takes 9.5 ms with them and 5.7 ms without (FP64, n = 64, 800 points),
     // 25.0 and 16.1 ms (int8, n = 128, 800 points), 5.3 and 4.4 ms (int8, n = 101, 312 points)
     const int symmetry = p.chol ? cholesky_symmetry(d) : 0;
@@ -444,7 +444,8 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
             set_error(PHF_ERR_UNSUPPORTED, "exchange_symmetry needs the FP64 form or n > 64 (tensor-core forms)");
             return PHF_ERR_UNSUPPORTED;
         }
-        p.ek_sym = sym_ok && d->exchange_symmetry != 2;
+        // (the tensor-core forms contract the Coulomb term over the pairs l <= j, the FP64 form over all (l, j))
+        p.ek_sym = sym_ok && d->exchange_symmetry != 2 && (p.prec == PHF_PREC_FP64 || symmetric);
         if (p.ek_sym) {
             // panels of indices i with Gram blocks (i n + l) x ((k >= i0) n + j) of at most ek_ipanel n x n^2
             const long long budget = (long long)p.ek_ipanel * n;
