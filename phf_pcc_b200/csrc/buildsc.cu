@@ -14,12 +14,17 @@
 // outer products and two-index contractions are the elementwise kernels below.  Tensors follow the
 // Fortran arrays: X(a, b, c, d) at a + M b + M^2 c + M^3 d, X(a, b) at a + M b.
 //
-// Everything between a point's four-index products and the sum over points is linear, so the weighted sums
-// over the points are taken first and the index permutations of t2 once at the end (one kernel over M^4
-// elements): sum_w s_w tau12_w and sum_w s_w tau20_w are single GEMMs with the contraction over (point, e), and
-// the outer products sum_w s_w Y_w (x) Z_w are GEMMs with the points as the contraction index.  Per point only
-// the four-index products, tau19 and two contractions remain.  (Assembling t2 point by point took 28 of the
-// 44 ms of 112 points at M = 32, in 172 passes over M^4 elements; now the whole sequence takes 15.6 ms.)
+// t2 is antisymmetric in (a, b) and in (c, d), and so is every t2_w.  tau10 is antisymmetrised in both of its index
+// pairs before the next two products take it, so that tau11 and tau12 already carry the antisymmetry:
+//   t2_w(a,b,c,d) = tau12(a,b,c,d) + tau11(a,c,d,b) - tau11(b,c,d,a) + tau10(c,d,a,b)
+//                   + Y(a,c) U(b,d) - Y(b,c) U(a,d) + Y(b,d) V(a,c) - Y(a,d) V(b,c)
+//   U(x,y) = tau8 Y(x,y) - tau18(x,y) + tau17(y,x) + q(y,x),  V(x,y) = tau27(y,x) + q(y,x),  q = tau21 - tau15
+// (tau20 of the sequence is tau11 of the antisymmetrised tau10).  Near a singular overlap Y goes as 1 / sigma and
+// these parts as its fourth power while det S t2_w stays bounded: antisymmetrising tau10 first removes the powers
+// before they are multiplied up, and the parts of a point are added before the weighted sum over the points takes
+// them.  (Weighted sums of each part over the points, antisymmetrised at the end: 1.7 times the error of the
+// sequence as it stands, as a geometric mean over 140 problems with n = 3..6, and up to twelve times; now 0.31.)
+// Assembling t2 point by point in 172 passes over M^4 elements took 28 of the 44 ms of 112 points at M = 32.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -62,41 +67,120 @@ __global__ void axpy4_kernel(int n0, int n1, int n2, int n3, int b, zc *out, S4 
     }
 }
 
-// out(a, b, c, d)_w = in(a, b, d, c)_w - in(a, b, c, d)_w
-__global__ void swap_last_kernel(int M, long long n, const zc *__restrict__ in, zc *__restrict__ out) {
-    const long long M2 = (long long)M * M;
-    for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < n; e += (long long)gridDim.x * NT) {
-        const long long ab = e % M2, r = e / M2;  // r = c + M d + M^2 w
-        const int c = (int)(r % M), d = (int)((r / M) % M);
-        out[e] = in[ab + M2 * (r + (long long)(d - c) + (long long)M * (c - d))] - in[e];
+// pair (e, f), e <= f, number p in the order of f
+__device__ __forceinline__ void pair_of(long long p, int &e, int &f) {
+    f = (int)((sqrt(8.0 * (double)p + 1.0) - 1.0) * 0.5);
+    while ((long long)f * (f + 1) / 2 > p) --f;
+    while ((long long)(f + 1) * (f + 2) / 2 <= p) ++f;
+    e = (int)(p - (long long)f * (f + 1) / 2);
+}
+
+// out = in antisymmetrised in (a, b) and in (c, d), a point per blockIdx.z: a block takes the planes (c, d) and (d, c)
+// of blockIdx.x's pair and the 32 x 32 tiles (I, J), (J, I) of (a, b), so that every row is read and written whole.
+constexpr int AT = 32, AT_P = AT + 1;
+__global__ void __launch_bounds__(NT) antisymmetrise_kernel(int M, const zc *__restrict__ in, zc *__restrict__ out) {
+    __shared__ zc s1[AT * AT_P], s2[AT * AT_P];
+    const long long M1 = M, M2 = M1 * M, M3 = M2 * M, base = blockIdx.z * M2 * M2;
+    int c, d, I, J;
+    pair_of(blockIdx.x, c, d);
+    pair_of(blockIdx.y, I, J);
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const zc *cd = in + base + M2 * c + M3 * d, *dc = in + base + M2 * d + M3 * c;
+    for (int q = ty; q < AT; q += NT / 32) {
+        const int a = I * AT + lane, b = J * AT + q, a2 = J * AT + lane, b2 = I * AT + q;
+        if (a < M && b < M) s1[q * AT_P + lane] = cd[a + M1 * b] - dc[a + M1 * b];
+        if (a2 < M && b2 < M) s2[q * AT_P + lane] = cd[a2 + M1 * b2] - dc[a2 + M1 * b2];
+    }
+    __syncthreads();
+    zc *ocd = out + base + M2 * c + M3 * d, *odc = out + base + M2 * d + M3 * c;
+    for (int q = ty; q < AT; q += NT / 32) {
+        const int a = I * AT + lane, b = J * AT + q, a2 = J * AT + lane, b2 = I * AT + q;
+        if (a < M && b < M) {
+            const zc v = s1[q * AT_P + lane] - s2[lane * AT_P + q];
+            ocd[a + M1 * b] = v;
+            if (c != d) odc[a + M1 * b] = mkz(-v.x, -v.y);
+        }
+        if (I != J && a2 < M && b2 < M) {
+            const zc v = s2[q * AT_P + lane] - s1[lane * AT_P + q];
+            ocd[a2 + M1 * b2] = v;
+            if (c != d) odc[a2 + M1 * b2] = mkz(-v.x, -v.y);
+        }
     }
 }
 
-// t2 from the weighted sums over the points: s12 = sum s tau12, s20 = sum s tau20, s10 = sum s tau10 and, at
-// (x + M y) + M^2 (p + M q), g = sum s Y(x, y) Z(p, q) for Z = tau8 Y - tau18 + tau17^T (g1), tau27, tau15, tau21:
-//   tau16 = s12 - g15[(a, c), (d, b)],   tau22 = -s20 + g21[(a, b), (c, d)]
-// divided by the projected overlap.
-__global__ void assemble_t2_kernel(int M, const zc *__restrict__ ovlp, const zc *__restrict__ s12, const zc *__restrict__ s20,
-                                   const zc *__restrict__ s10, const zc *__restrict__ g1, const zc *__restrict__ g27,
-                                   const zc *__restrict__ g15, const zc *__restrict__ g21, zc *__restrict__ t2) {
+// acc(a, b, c, d) += sum_w s_w [t12(a,b,c,d) + t11(a,c,d,b) - t11(b,c,d,a) + Y(a,c) U(b,d) - Y(b,c) U(a,d) + Y(b,d) V(a,c)
+// - Y(a,d) V(b,c)]_w for c <= d and the tiles of 32 a and 8 b that reach a <= b.  A warp of the block takes every
+// eighth point (t11(b,c,d,a) through its own 8 x 32 tile of shared memory), the warps' sums are added in order:
+// one warp for all points was a chain of as many load latencies as points.
+// Bound: t11 and a quarter of t12 read once (M = 32, 112 points: 1.9 GB in all).
+constexpr int PT_B = 8, PT_W = NT / 32;
+__global__ void __launch_bounds__(NT) points_t2_kernel(int M, int b, const zc *__restrict__ t12, const zc *__restrict__ t11,
+                                                       const zc *__restrict__ Y, const zc *__restrict__ U,
+                                                       const zc *__restrict__ V, const zc *__restrict__ sc,
+                                                       zc *__restrict__ acc) {
+    __shared__ zc tr[PT_W][PT_B * AT_P], col[PT_W][4][PT_B];
+    const long long M1 = M, M2 = M1 * M, M3 = M2 * M, M4 = M2 * M2;
+    int c, d;
+    pair_of(blockIdx.x, c, d);
+    const int nb = (M + PT_B - 1) / PT_B, a0 = (int)(blockIdx.y / nb) * AT, b0 = (int)(blockIdx.y % nb) * PT_B;
+    if (a0 >= b0 + PT_B) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, a = a0 + lane, rb = lane % PT_B, ra = lane / PT_B;
+    zc v[PT_B];
+#pragma unroll
+    for (int q = 0; q < PT_B; ++q) v[q] = mkz(0, 0);
+    for (int w = wid; w < b; w += PT_W) {
+        const zc *T = t11 + w * M4 + M1 * c + M2 * d, *y = Y + w * M2, *u = U + w * M2, *x = V + w * M2;
+        __syncwarp();
+        if (b0 + rb < M) {
+#pragma unroll
+            for (int k = 0; k < PT_B; ++k) {  // element (b, a) at tr[b][a]
+                const int ka = ra + 4 * k;
+                if (a0 + ka < M) tr[wid][rb * AT_P + ka] = T[b0 + rb + M3 * (a0 + ka)];
+            }
+            const zc *src = ra == 0 ? y + M1 * c : (ra == 1 ? y + M1 * d : (ra == 2 ? u + M1 * d : x + M1 * c));
+            col[wid][ra][rb] = src[b0 + rb];
+        }
+        __syncwarp();
+        if (a < M) {
+            const zc yc = y[a + M1 * c], yd = y[a + M1 * d], ud = u[a + M1 * d], vc = x[a + M1 * c], s = sc[w];
+#pragma unroll
+            for (int q = 0; q < PT_B; ++q) {
+                const int bb = b0 + q;
+                if (bb < M) {
+                    zc t = t12[w * M4 + a + M1 * bb + M2 * c + M3 * d] + (T[a + M3 * bb] - tr[wid][q * AT_P + lane]);
+                    t = t + (yc * col[wid][2][q] - col[wid][0][q] * ud + col[wid][1][q] * vc - yd * col[wid][3][q]);
+                    v[q] = v[q] + s * t;
+                }
+            }
+        }
+    }
+    for (int k = 0; k < PT_W; ++k) {  // (tr of warp 0 holds the running sum)
+        __syncthreads();
+        if (wid == k) {
+#pragma unroll
+            for (int q = 0; q < PT_B; ++q) tr[0][q * AT_P + lane] = k ? tr[0][q * AT_P + lane] + v[q] : v[q];
+        }
+    }
+    if (wid == PT_W - 1 && a < M) {
+        for (int q = 0; q < PT_B; ++q)
+            if (b0 + q < M) {
+                zc *o = acc + a + M1 * (b0 + q) + M2 * c + M3 * d;
+                *o = *o + tr[0][q * AT_P + lane];
+            }
+    }
+}
+
+// t2 = (acc(a, b, c, d) + s10(c, d, a, b)) / overlap from the elements a <= b, c <= d by antisymmetry
+__global__ void finish_t2_kernel(int M, const zc *__restrict__ ovlp, const zc *__restrict__ acc, const zc *__restrict__ s10,
+                                 zc *__restrict__ t2) {
     const long long M1 = M, M2 = M1 * M, M3 = M2 * M, M4 = M2 * M2;
     const zc ov = *ovlp;
     for (long long e = blockIdx.x * (long long)NT + threadIdx.x; e < M4; e += (long long)gridDim.x * NT) {
         const long long a = e % M, b = (e / M) % M, c = (e / M2) % M, d = e / M3;
-        const auto at = [&](const zc *X, long long i, long long j, long long k, long long l) {
-            return X[i + M1 * j + M2 * k + M3 * l];
-        };
-        const auto t16 = [&](long long i, long long j, long long k, long long l) {
-            return at(s12, i, j, k, l) - at(g15, i, k, l, j);
-        };
-        const auto t22 = [&](long long i, long long j, long long k, long long l) {
-            return at(g21, i, j, k, l) - at(s20, i, j, k, l);
-        };
-        zc v = at(g1, a, c, b, d) - at(g1, b, c, a, d);
-        v = v + (at(g27, b, d, c, a) - at(g27, a, d, c, b));
-        v = v + (t16(a, b, c, d) - t16(a, b, d, c) - t16(b, a, c, d) + t16(b, a, d, c));
-        v = v + (t22(a, c, d, b) - t22(a, d, c, b) - t22(b, c, d, a) + t22(b, d, c, a));
-        v = v + (at(s10, c, d, a, b) - at(s10, c, d, b, a) - at(s10, d, c, a, b) + at(s10, d, c, b, a));
+        const long long a1 = min(a, b), b1 = max(a, b), c1 = min(c, d), d1 = max(c, d);
+        zc v = acc[a1 + M1 * b1 + M2 * c1 + M3 * d1] + s10[c1 + M1 * d1 + M2 * a1 + M3 * b1];
+        if (a == b || c == d) v = v - v;  // zero, or not a number
+        if ((a > b) != (c > d)) v = mkz(-v.x, -v.y);
         t2[e] = divz(v, ov);
     }
 }
@@ -224,15 +308,6 @@ struct Ctx {
         PHF_CHECK_LAUNCH();
         return PHF_OK;
     }
-    // acc(a, b, c, d) += sum over the points and e of Ys(a, e) X(b, c, d, e): one GEMM, contraction (point, e)
-    int gemm4_sum(zc *acc, const zc *Ys, const zc *X) const {
-        return zgemm_strided((int)M3(), M, M * b, 1, 1, ONE, V(X, 1, M3()), V(Ys, M, 1), ONE, O(acc, M, 1), nullptr, st);
-    }
-    // acc[(x, y), (p, q)] += sum over the points of Ys(x, y) Z(p, q)
-    int outer_sum(zc *acc, const zc *Ys, const zc *Z) const {
-        return zgemm_strided((int)M2(), (int)M2(), b, 1, 1, ONE, V(Ys, 1, M2()), V(Z, M2(), 1), ONE, O(acc, 1, M2()),
-                             nullptr, st);
-    }
     // out_w (+)= sign sum_{a,b} X(a, b) Z(a, b) or Z(b, a)
     int trace2(zc *out, const zc *X, const zc *Z, bool transposed, double sign, int init) const {
         trace2_kernel<<<b, NT, 0, st>>>(M, out, X, Z, transposed ? M : 1, transposed ? 1 : M, M2(), sign, init);
@@ -330,8 +405,8 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     // chunk workspace
     zc *T = nullptr, *R = nullptr, *Sinv = nullptr, *det = nullptr, *logdet = nullptr, *Y = nullptr, *c1t = nullptr,
        *t2d = nullptr, *sc = nullptr, *sclr = nullptr, *acc0 = nullptr, *acc1 = nullptr, *acc2 = nullptr,
-       *ovlp = nullptr;
-    zc *B4[3] = {}, *S4sum[7] = {};  // weighted sums over the points: s12, s20, s10, g1, g27, g15, g21
+       *s10 = nullptr, *ovlp = nullptr;
+    zc *B4[3] = {};
     zc *B2[18] = {};
     int *flag = nullptr;
     PHF_TRY(ar.alloc(&T, (size_t)b * M2));
@@ -345,7 +420,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     PHF_TRY(ar.alloc(&sc, (size_t)b));
     PHF_TRY(ar.alloc(&sclr, 4 * (size_t)b));
     for (auto &p : B4) PHF_TRY(ar.alloc(&p, (size_t)b * M4));
-    for (auto &p : S4sum) PHF_TRY(ar.alloc(&p, (size_t)M4));
+    PHF_TRY(ar.alloc(&s10, (size_t)M4));  // sum over the points of s tau10
     for (auto &p : B2) PHF_TRY(ar.alloc(&p, (size_t)b * M2));
     PHF_TRY(ar.alloc(&acc0, 1));
     PHF_TRY(ar.alloc(&acc1, (size_t)M2));
@@ -355,14 +430,15 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
     cudaStream_t st = 0;
     PHF_CUDA(cudaMemsetAsync(acc0, 0, sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(acc1, 0, M2 * sizeof(zc), st));
-    for (auto &p : S4sum) PHF_CUDA(cudaMemsetAsync(p, 0, M4 * sizeof(zc), st));
+    PHF_CUDA(cudaMemsetAsync(acc2, 0, M4 * sizeof(zc), st));
+    PHF_CUDA(cudaMemsetAsync(s10, 0, M4 * sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(ovlp, 0, sizeof(zc), st));
     PHF_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
     // four-index buffers (reused as the sequence allows) and two-index intermediates
-    zc *c2t = B4[0], *tau11 = B4[0], *tmp = B4[1], *tau9 = B4[1], *tau19 = B4[1], *tau10 = B4[2];
+    zc *c2t = B4[0], *tmp = B4[1], *tau9 = B4[1], *tau10 = B4[0], *tau10a = B4[1], *tau11 = B4[0], *tau12 = B4[2];
     zc *tau1 = B2[0], *tau2 = B2[1], *tau5 = B2[2], *tau6 = B2[3], *tau7 = B2[4], *tau13 = B2[5], *tau14 = B2[6],
        *tau15 = B2[7], *tau17 = B2[8], *tau18 = B2[9], *tau21 = B2[10], *tau24 = B2[11], *tau25 = B2[12],
-       *tau26 = B2[13], *tau27 = B2[14], *a1 = B2[15], *Ys = B2[16], *Z1 = B2[17];
+       *tau26 = B2[13], *tau27 = B2[14], *a1 = B2[15], *U = B2[16], *V2 = B2[17];
     zc *tau3 = sclr, *tau8 = sclr + b, *tau23 = sclr + 2 * (size_t)b, *a0 = sclr + 3 * (size_t)b;
     const zc c0{c0h.re, c0h.im};
 
@@ -395,11 +471,10 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
                               nullptr, st));  // (i,j,k,l) = sum_x conj U(x,i) (x,j,k,l)
 
         // ---- BuildSC_Vec (PHF_fort/BuildSC_dr.f90), Y = the transition density of each point
-        // weights s_w = det S_w weightsp wpg (...) of the points, and s_w Y_w
+        // weights s_w = det S_w weightsp wpg (...) of the points
         weights_kernel<<<(bc + NT - 1) / NT, NT, 0, st>>>(bc, w0, det, wtd, sc, ovlp);
         ++g_launches;
         PHF_CHECK_LAUNCH();
-        PHF_TRY(x.axpy2(Ys, Y, false, 1.0, 1, sc));
         // tau0(a,b,c,d) = c2(a,b,c,d) - c2(b,a,c,d), read in place
         PHF_TRY(x.contract2(tau1, Y, c2t, "dabc", "adbc"));                  // tau1 = Y(c,d) tau0(d,a,b,c)
         PHF_TRY(x.axpy2(tau2, tau1, false, -1.0, 1));
@@ -424,20 +499,15 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         PHF_TRY(x.gemm2(a1, V(tau7, 1, M, M2), V(Y, 1, M, M2), MONE, ONE));  // - Y(c,b) tau7(a,c)
         PHF_TRY(x.gemm4(tau9, Y, false, c2t));                                // Y(e,a) c2(b,c,d,e)
         PHF_TRY(x.gemm4(tau10, Y, false, tau9));                              // Y(e,a) tau9(b,c,d,e)
-        PHF_TRY(x.gemm4(tau11, Y, true, tau10));                              // Y(a,e) tau10(b,c,d,e)
-        PHF_TRY(x.gemm4_sum(S4sum[0], Ys, tau11));                            // s12: tau12 = Y(a,e) tau11(b,c,d,e)
-        swap_last_kernel<<<blocks_for(M4 * bc), NT, 0, st>>>(M, M4 * bc, tau10, tau19);  // tau10(abdc) - tau10(abcd)
-        ++g_launches;
+        const unsigned npair = (unsigned)(M2 + M) / 2, ntile = (unsigned)((M + AT - 1) / AT);
+        antisymmetrise_kernel<<<dim3(npair, ntile * (ntile + 1) / 2, (unsigned)bc), NT, 0, st>>>(M, tau10, tau10a);
+        accumulate_kernel<<<blocks_for(M4), NT, 0, st>>>(M4, bc, tau10a, sc, s10);
+        g_launches += 2;
         PHF_CHECK_LAUNCH();
-        PHF_TRY(x.gemm4_sum(S4sum[1], Ys, tau19));                            // s20: tau20 = Y(a,e) tau19(b,c,d,e)
-        accumulate_kernel<<<blocks_for(M4), NT, 0, st>>>(M4, bc, tau10, sc, S4sum[2]);  // s10
-        ++g_launches;
-        PHF_CHECK_LAUNCH();
+        PHF_TRY(x.gemm4(tau11, Y, true, tau10a));                             // Y(a,e) tau10(b,c,d,e)
+        PHF_TRY(x.gemm4(tau12, Y, true, tau11));                              // Y(a,e) tau11(b,c,d,e)
         PHF_TRY(x.gemm2(tau17, V(Y, M, 1, M2), V(c1t, M, 1, M2)));           // Y(c,a) c1(b,c)
         PHF_TRY(x.gemm2(tau18, V(Y, 1, M, M2), V(tau17, M, 1, M2)));         // Y(a,c) tau17(b,c)
-        PHF_TRY(x.axpy2(Z1, Y, false, 1.0, 1, tau8));                         // tau8 Y(b,d) - tau18(b,d) + tau17(d,b)
-        PHF_TRY(x.axpy2(Z1, tau18, false, -1.0, 0));
-        PHF_TRY(x.axpy2(Z1, tau17, true, 1.0, 0));
         PHF_TRY(x.trace2(tau23, Y, c1t, true, 1.0, 1));                       // tau23 = Y(b,a) c1(a,b)
         PHF_TRY(x.axpy2(tau27, Y, true, 1.0, 1, tau23));                      // tau27 = tau23 Y(b,a)
         PHF_TRY(x.gemm2(tau24, V(Y, 1, M, M2), V(c1t, 1, M, M2)));           // Y(a,c) c1(c,b)
@@ -457,8 +527,17 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
             ++g_launches;
             PHF_CHECK_LAUNCH();
         }
-        const zc *Zs[4] = {Z1, tau27, tau15, tau21};
-        for (int z = 0; z < 4; ++z) PHF_TRY(x.outer_sum(S4sum[3 + z], Ys, Zs[z]));
+        PHF_TRY(x.axpy2(tau21, tau15, false, -1.0, 0));                       // q = tau21 - tau15
+        PHF_TRY(x.axpy2(U, Y, false, 1.0, 1, tau8));                          // tau8 Y - tau18 + tau17^T + q^T
+        PHF_TRY(x.axpy2(U, tau18, false, -1.0, 0));
+        PHF_TRY(x.axpy2(U, tau17, true, 1.0, 0));
+        PHF_TRY(x.axpy2(U, tau21, true, 1.0, 0));
+        PHF_TRY(x.axpy2(V2, tau27, true, 1.0, 1));                            // tau27^T + q^T
+        PHF_TRY(x.axpy2(V2, tau21, true, 1.0, 0));
+        points_t2_kernel<<<dim3(npair, ntile * (unsigned)((M + PT_B - 1) / PT_B)), NT, 0, st>>>(M, bc, tau12, tau11, Y, U,
+                                                                                            V2, sc, acc2);
+        ++g_launches;
+        PHF_CHECK_LAUNCH();
 
         // ---- accumulation of the smaller parts over the chunk's points (fixed order)
         accumulate_kernel<<<1, NT, 0, st>>>(1, bc, a0, sc, acc0);
@@ -466,8 +545,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         g_launches += 2;
         PHF_CHECK_LAUNCH();
     }
-    assemble_t2_kernel<<<blocks_for(M4), NT, 0, st>>>(M, ovlp, S4sum[0], S4sum[1], S4sum[2], S4sum[3], S4sum[4], S4sum[5],
-                                                      S4sum[6], acc2);
+    finish_t2_kernel<<<blocks_for(M4), NT, 0, st>>>(M, ovlp, acc2, s10, B4[0]);
     ++g_launches;
     PHF_CHECK_LAUNCH();
     std::vector<cd> h0(1), h1(M2), ho(1);
@@ -494,7 +572,7 @@ int buildsc_run(phf_complex c0h, const phf_complex *c1h, const phf_complex *c2h,
         t1h[i].re = v.real();
         t1h[i].im = v.imag();
     }
-    PHF_CUDA(cudaMemcpy(t2h, acc2, M4 * sizeof(zc), cudaMemcpyDeviceToHost));
+    PHF_CUDA(cudaMemcpy(t2h, B4[0], M4 * sizeof(zc), cudaMemcpyDeviceToHost));
     return PHF_OK;
 }
 
