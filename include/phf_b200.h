@@ -335,6 +335,11 @@ int phf_int8_wide_mma(int on);
    as slices, k = 2M) instead of an FP64 GEMM per point; 0 keeps the FP64 product; a value above 1 also caps the points per sub-batch of that GEMM
    (otherwise sized to 1 GiB of slices).  Returns the previous setting.  No counterpart in the reference. */
 int phf_int8_fock_product(int on);
+/* The one-shot calls (phf_buildhsg, phf_buildhsg_chol, phf_localg, phf_buildsc, phf_pbarhbarolap) keep the device
+   memory they used for the next one: at most 16 GiB and at most half of what is free when a call ends.  A
+   cudaMalloc of the same process that would fail gets it; this returns the current device's to the driver, for
+   other processes and for what counts the free memory. */
+void phf_release_memory(void);
 /* Library version string. */
 const char *phf_version(void);
 

@@ -194,6 +194,12 @@ def buildsc(c0, c1, c2, nocc, ngrid, qj, r1, r2, rpg, rk, roota, rootb, rooty, w
     return complex(t0.re, t0.im), t1, t2
 
 
+def release_memory() -> None:
+    """Return the device memory that one-shot calls keep for the next one (at most 16 GiB) to the driver, for
+    other processes (a cudaMalloc of this process that would fail gets it without this call)."""
+    _lib.load().phf_release_memory()
+
+
 def pbarhbarolap(hone, htwo, ref, t1, t2, nocc, nao, nso, enuc, qj, sp, npoints, npg, ncisp, ncipg, ncik, r1, r2,
                  rpg, rk, roota, rootb, rooty, weightsp, weightpg, fsp, fpg, fk, trunode, comm=None, workspace=0):
     """PbarHbarOlap (SUCCSD_Boson_cmplx/FPUCC.f90:14-272), the projected-CCSD grid kernel, on the GPU.

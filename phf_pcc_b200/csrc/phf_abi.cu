@@ -365,6 +365,8 @@ int phf_profile_read(int kernel_class, double *total_ms, unsigned long long *lau
     return phf::profile_read(kernel_class, total_ms, launches);
 }
 
+void phf_release_memory(void) { phf::pool_release(); }
+
 const char *phf_version(void) { return kVersion; }
 
 }  // extern "C"

@@ -117,7 +117,10 @@ cudaMemPool_t g_pools[kPoolDevices] = {};  // one per device, created at first u
 
 cudaMemPool_t current_pool(bool create) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) return nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) {
+        cudaGetLastError();
+        return nullptr;
+    }
     std::lock_guard<std::mutex> lock(g_pool_mu);
     if (!g_pools[dev] && create) {
         cudaMemPoolProps props = {};
@@ -143,8 +146,7 @@ cudaError_t pool_alloc(void **p, size_t bytes) {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, 0);
     if (e == cudaErrorMemoryAllocation) {  // give back what is kept and try once more
         cudaGetLastError();
-        cudaStreamSynchronize(0);
-        cudaMemPoolTrimTo(pool, 0);
+        pool_release();
         e = cudaMallocFromPoolAsync(p, bytes, pool, 0);
     }
     return e;
@@ -152,18 +154,42 @@ cudaError_t pool_alloc(void **p, size_t bytes) {
 
 void pool_free(void *p) { cudaFreeAsync(p, 0); }
 
+namespace {
+// bytes held by the pool and in use of it (no pool: zero)
+void pool_bytes(cudaMemPool_t pool, size_t &held, size_t &used) {
+    unsigned long long h = 0, u = 0;
+    if (pool) {
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &h);
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &u);
+    }
+    held = (size_t)h;
+    used = (size_t)std::min(u, h);
+}
+}  // namespace
+
+size_t pool_kept_bytes() {
+    size_t held, used;
+    pool_bytes(current_pool(false), held, used);
+    return held - used;
+}
+
+void pool_release() {
+    cudaMemPool_t pool = current_pool(false);
+    if (!pool) return;
+    cudaStreamSynchronize(0);  // frees that are queued there
+    cudaMemPoolTrimTo(pool, 0);
+}
+
 void pool_trim() {
     cudaMemPool_t pool = current_pool(false);
-    size_t fr = 0, tot = 0;
+    size_t fr = 0, tot = 0, held, used;
     if (!pool || cudaMemGetInfo(&fr, &tot) != cudaSuccess) return;
-    unsigned long long held = 0, used = 0;
-    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held);
-    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    pool_bytes(pool, held, used);
     // keep at most half of what would be free without the kept part
-    const size_t keep = std::min(kPoolKeep, (fr + (size_t)(held - used)) / 2);
+    const size_t keep = std::min(kPoolKeep, (fr + (held - used)) / 2);
     if (held - used > keep) {
         cudaStreamSynchronize(0);
-        cudaMemPoolTrimTo(pool, (size_t)used + keep);
+        cudaMemPoolTrimTo(pool, used + keep);
     }
 }
 
@@ -716,7 +742,8 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
         size_t budget = d->workspace_bytes ? d->workspace_bytes : ((size_t)6 << 30);
         if (!d->workspace_bytes && p.streamed) {
             size_t fr = 0, tot = 0;
-            if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) budget = std::max(budget, (size_t)(0.45 * (double)fr));
+            if (cudaMemGetInfo(&fr, &tot) == cudaSuccess)  // (what is kept for one-shot calls can be had, too)
+                budget = std::max(budget, (size_t)(0.45 * (double)(fr + pool_kept_bytes())));
             cudaGetLastError();
         }
         size_t per = 5 * MN + 3 * (size_t)N * N + 8;

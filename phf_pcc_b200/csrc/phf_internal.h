@@ -21,14 +21,17 @@ struct DevBuf {
 // Device memory of calls that allocate and free within themselves (one-shot buildhsg, localg, BuildSC, the
 // projected-CC kernel): a stream-ordered pool per device, on the legacy default stream, which is where those
 // calls run.  It keeps freed memory for the next call, at most 16 GiB and at most half of what is free on the
-// device when a call ends (pool_trim), and gives the rest back to the driver; a failed allocation gives all of it
-// back first.  Safe for several threads: the pool is the driver's, and every use is ordered on the one stream.
+// device when a call ends (pool_trim).  The driver takes it back for a cudaMalloc of this process that
+// would fail otherwise (a plan's, another allocator's), pool_alloc gives it back before it tries once more, and
+// phf_release_memory does so for other processes.  Safe for several threads: the pool is the driver's, and every
+// use is ordered on the one stream.
 // (With cudaMalloc and cudaFree in every call: projected-CC kernel, M = 40, 92 ms against 50; BuildSC, M = 32, 49
-// against 20, ten of them the division by the overlap on the host; dense buildhsg, M = 40, 8.2 against 4.9, a part
-// of it a CUDA graph captured for one evaluation.)
+// against 20, ten of them the division by the overlap on the host.)
 cudaError_t pool_alloc(void **p, size_t bytes);
 void pool_free(void *p);
-void pool_trim();  // at the end of a call
+void pool_trim();          // at the end of a call
+void pool_release();       // everything that is not in use
+size_t pool_kept_bytes();  // held on the current device and not in use
 
 struct Arena {
     std::vector<DevBuf> bufs;
