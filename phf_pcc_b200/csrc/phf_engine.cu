@@ -1806,7 +1806,12 @@ void plan_release(PlanImpl &p) {
         }
     if (p.ev_fork) cudaEventDestroy(p.ev_fork);
     if (p.ev_join) cudaEventDestroy(p.ev_join);
-    if (p.side) cudaStreamDestroy(p.side);
+    if (p.side) {
+        // an evaluation that failed between the fork and the join leaves work here, and pooled memory (one-shot
+        // calls) is reused in the order of the legacy default stream, which does not wait for this stream
+        cudaStreamSynchronize(p.side);
+        cudaStreamDestroy(p.side);
+    }
     p.ev_fork = p.ev_join = nullptr;
     p.side = nullptr;
     if (p.cap_stream) {
