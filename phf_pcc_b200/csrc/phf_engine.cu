@@ -372,6 +372,29 @@ int choose_ipanel(int n) {
 }  // namespace
 
 namespace {
+// Residues of the products of a chunk of b points: of one exchange product over `points` of them (all, or equal parts
+// of at most 1 GiB, whole 256-row tiles) and of the larger of the Coulomb products.  Returned: a bound of the bytes that
+// does not fall as b grows.
+struct RzScratch {
+    long long points;
+    size_t c, cj;
+};
+size_t rz_scratch(const PlanImpl &p, long long b, RzScratch *out) {
+    const size_t tile = rz_product_bytes(2 * kRzModuli, 1, p.rz_rows);
+    const long long groups = (b + 31) / 32, cap = std::max<long long>(1, (long long)(((size_t)1 << 30) / tile));
+    const auto coulomb = [&](long long points) {
+        return std::max(rz_product_bytes(kRzModuli, 2 * points, p.rz_rows), rz_product_bytes(kRzModuli, 2 * b, p.L));
+    };
+    if (out) {
+        const long long parts = (groups + cap - 1) / cap;
+        out->points = std::min(b, 32 * ((groups + parts - 1) / parts));
+        out->c = rz_product_bytes(2 * kRzModuli, 8 * out->points, p.rz_rows);
+        out->cj = coulomb(out->points);
+    }
+    const long long most = std::min(groups, cap);
+    return tile * (size_t)most + coulomb(32 * most);
+}
+
 // How the Cholesky vectors compare with their transposes (16 x 16 tiles, so that both sides stay in cache): 2 = every
 // B_L is exactly symmetric, 1 = to rounding, 0 = neither (or not finite).  To rounding: no difference above 2 sqrt(n)
 // units in the last place of the largest element of B_L.  Vectors brought to another basis, X^T B X, are sums of n
@@ -752,14 +775,14 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
             per += MM;                                          // Rho and Gam
             if (!p.rz) per += 2 * n2 + p.L;                     // Pvec, Jvec, dvec
             if (p.prec == PHF_PREC_FP64) per += 8 * n2;         // Kin, Kvec
-            else if (p.rz) per += (rz_operand_bytes(2 * kRzModuli, 8, n * (n + 1) / 2) + rz_operand_bytes(kRzModuli, 2, n * (n + 1) / 2) +
-                                   2 * rz_operand_bytes(kRzModuli, 2, p.L)) / sizeof(zc) + 1;  // the operands and d
+            else if (p.rz)  // the operands (their products are counted below)
+                per += (rz_operand_bytes(2 * kRzModuli, 8, n * (n + 1) / 2) + rz_operand_bytes(kRzModuli, 2, n * (n + 1) / 2) +
+                        rz_operand_bytes(kRzModuli, 2, p.L)) / sizeof(zc) + 2;
             else per += (8 * (n2 + 64) * oz_slots(p.slices)) / sizeof(zc) + 1  // exchange slices
                         + (2 * n2 + 2 * (size_t)p.L) * oz_slots(p.slices) / sizeof(zc) + 1    // Coulomb slices
                         + p.L + n2;                                                // d^T, J pairs
-            // int8 density GEMM: the X rows' slices and exponents (counted for n <= 128 too, where the residue form
-            // does without: a given workspace makes the same chunks)
-            if (p.prec != PHF_PREC_FP64 && !oz_rho_slice_ok(n) && p.slices <= 7) {
+            // int8 density GEMM: the X rows' slices and exponents
+            if (p.prec != PHF_PREC_FP64 && density_i8(p)) {
                 per += ((size_t)M * oz_pad_k(2LL * N) * oz_slots(p.slices) + 4 * (size_t)M) / sizeof(zc) + 1;
                 // F X on the int8 path: the slices and exponents of X's columns and F's rows
                 if (g_fx_i8 && oz_fx_ok(M, p.slices))
@@ -775,6 +798,15 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
         per *= sizeof(zc);
         long long bmax = (long long)(budget / std::max<size_t>(per, 1));
         bmax = std::max<long long>(1, std::min<long long>(bmax, 4096));
+        if (p.rz) {  // the largest chunk whose residue products fit too
+            long long lo = 1, hi = bmax;
+            while (lo < hi) {
+                const long long mid = (lo + hi + 1) / 2;
+                if (per * (size_t)mid + rz_scratch(p, mid, nullptr) <= budget) lo = mid;
+                else hi = mid - 1;
+            }
+            bmax = lo;
+        }
         p.b = (int)std::min<long long>(bmax, p.wend - p.wbeg);
         // whole Lebedev-point blocks (ny npg points sharing R1[il]) per chunk when they fit
         const int blk = p.ny * p.npg;
@@ -826,14 +858,11 @@ int plan_create(const phf_plan_desc *d, phf_plan **out, bool one_shot) {
                 PHF_TRY(p.arena.alloc(&p.rzPe, 2 * b));
                 PHF_TRY(p.arena.alloc(&p.rzD, rz_operand_bytes(kRzModuli, 2LL * b, p.L)));
                 PHF_TRY(p.arena.alloc(&p.rzDe, 2 * b));
-                // residues of one product: all points, or equal parts of at most 1 GiB (whole 256-row tiles)
-                const size_t tile = rz_product_bytes(2 * kRzModuli, 1, p.rz_rows);
-                const long long groups = (p.b + 31) / 32, cap = std::max<long long>(1, (long long)(((size_t)1 << 30) / tile));
-                const long long parts = (groups + cap - 1) / cap;
-                p.rz_sub = (int)std::min<long long>(p.b, 32 * ((groups + parts - 1) / parts));
-                PHF_TRY(p.arena.alloc(&p.rzC, rz_product_bytes(2 * kRzModuli, 8LL * p.rz_sub, p.rz_rows)));
-                PHF_TRY(p.arena.alloc(&p.rzCJ, std::max(rz_product_bytes(kRzModuli, 2LL * p.rz_sub, p.rz_rows),
-                                                        rz_product_bytes(kRzModuli, 2LL * b, p.L))));
+                RzScratch sz;
+                rz_scratch(p, p.b, &sz);
+                p.rz_sub = (int)sz.points;
+                PHF_TRY(p.arena.alloc(&p.rzC, sz.c));
+                PHF_TRY(p.arena.alloc(&p.rzCJ, sz.cj));
             } else {
                 const long long npadK = oz_pad_cols(8 * (long long)b);
                 size_t bsl = oz_slice_bytes(npadK, (long long)n2, p.slices);
