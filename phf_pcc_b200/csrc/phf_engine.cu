@@ -1056,39 +1056,61 @@ int build_exchange_matrix(PlanImpl &p) {
         PHF_CUDA(cudaDeviceSynchronize());
         return PHF_OK;
     }
-    if (p.ek_sym) {  // the whole Gram block once, then the symmetric and antisymmetric rows of all pairs
-        const long long kks = (long long)n * (n + 1) / 2, kka = (long long)n * (n - 1) / 2;
+    if (p.ek_sym) {
+        // The symmetric and antisymmetric rows of all pairs from the Gram block, in panels of indices i of at most 1 GiB
+        // of it: the whole block is twice the FP64 rows kept (n = 128: 2.1 GB beside 1.1), and made a plan that fits
+        // run out of memory while it was formed.  (Slices take the whole block; it and they are less than the full
+        // rows and theirs.)
+        const long long kks = (long long)n * (n + 1) / 2, kka = (long long)n * (n - 1) / 2, nn = n;
+        const bool slices = p.prec != PHF_PREC_FP64 && !p.rz;
+        const int panel = slices ? n : (int)std::max<long long>(1, std::min(nn, (1LL << 27) / (nn * n2)));
+        const long long rs = oz_pad_rows(kks), ra = oz_pad_rows(kka);
+        size_t bs = 0;
         PHF_TRY(upload_pair_tables(p));
-        double *G = nullptr;
-        PHF_TRY(p.arena.alloc(&G, (size_t)(n2 * n2)));
-        OutView go = vo(reinterpret_cast<zc *>(G), n2, 1);
-        go.real = 1;
-        PHF_TRY(zgemm_strided((int)n2, (int)n2, L, 1, 1, Z1, vd(p.Bst, 1, n2), vd(p.Bst, n2, 1), Z0, go, nullptr, 0));
         if (p.prec == PHF_PREC_FP64) {
             PHF_TRY(p.arena.alloc(&p.EK, (size_t)(kks * kks + kka * kka)));
-            PHF_TRY(launch_ek_sym_panel(n, 0, n, 0, p.pairs_le, G, n2, p.EK, p.EK + kks * kks, 0));
-            // the Coulomb term over pairs: B_L[l][j] (2 - delta_lj)
-            PHF_TRY(p.arena.alloc(&p.Bpair, (size_t)(L * kks)));
-            PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, p.Bpair, 0));
         } else if (p.rz) {
             p.rz_rows = kks;
             PHF_TRY(p.arena.alloc(&p.rzE, rz_operand_bytes(2 * kRzModuli, kks, kks)));
             PHF_TRY(p.arena.alloc(&p.rzEe, (size_t)(2 * kks)));
-            PHF_TRY(rz_exchange_rows(n, 0, n, 0, p.pairs_le, G, n2, kks, p.rzE, p.rzEe, 0));
-            PHF_TRY(build_coulomb_slices(p));
         } else {
-            const long long rs = oz_pad_rows(kks), ra = oz_pad_rows(kka);
-            const size_t bs = oz_slice_bytes(rs, kks, p.slices), ba = oz_slice_bytes(ra, kka, p.slices);
+            bs = oz_slice_bytes(rs, kks, p.slices);
+            const size_t ba = oz_slice_bytes(ra, kka, p.slices);
             PHF_TRY(p.arena.alloc(&p.EKsl, bs + ba));
             PHF_CUDA(cudaMemset(p.EKsl, 0, bs + ba));
             PHF_TRY(p.arena.alloc(&p.ea, (size_t)(rs + ra)));
             PHF_CUDA(cudaMemset(p.ea, 0, (size_t)(rs + ra) * sizeof(int)));
-            PHF_TRY(oz_slice_ek_sym_panel(n, 0, n, 0, p.pairs_le, G, n2, p.slices, rs, p.EKsl, p.ea, ra, p.EKsl + bs,
-                                          p.ea + rs, 0));
-            PHF_TRY(build_coulomb_slices(p));
+        }
+        double *G = nullptr;
+        PHF_TRY(p.arena.alloc(&G, (size_t)(panel * nn * n2)));
+        for (int i0 = 0; i0 < n; i0 += panel) {
+            const int ip = std::min(panel, n - i0);
+            const long long gcols = (nn - i0) * nn, ts0 = pair_index_le(nn, i0, i0),
+                            ta0 = i0 + 1 < n ? pair_index_lt(nn, i0, i0 + 1) : kka;
+            OutView go = vo(reinterpret_cast<zc *>(G), gcols, 1);
+            go.real = 1;
+            PHF_TRY(zgemm_strided(ip * n, (int)gcols, L, 1, 1, Z1, vd(p.Bst + (size_t)i0 * n, 1, n2),
+                                  vd(p.Bst + (size_t)i0 * n, n2, 1), Z0, go, nullptr, 0));
+            if (p.prec == PHF_PREC_FP64)
+                PHF_TRY(launch_ek_sym_panel(n, i0, ip, i0, p.pairs_le, G, gcols, p.EK + ts0 * kks,
+                                            p.EK + kks * kks + ta0 * kka, 0));
+            else if (p.rz)
+                PHF_TRY(rz_exchange_rows(n, i0, ip, i0, p.pairs_le, G, gcols, kks,
+                                         p.rzE + (size_t)ts0 * rz_operand_bytes(1, 1, kks), p.rzEe + ts0, 0));
+            else
+                PHF_TRY(oz_slice_ek_sym_panel(n, 0, n, 0, p.pairs_le, G, n2, p.slices, rs, p.EKsl, p.ea, ra, p.EKsl + bs,
+                                              p.ea + rs, 0));
         }
         PHF_CUDA(cudaDeviceSynchronize());
         p.arena.free_one(G);
+        if (p.prec == PHF_PREC_FP64) {
+            // the Coulomb term over pairs: B_L[l][j] (2 - delta_lj)
+            PHF_TRY(p.arena.alloc(&p.Bpair, (size_t)(L * kks)));
+            PHF_TRY(oz_cholesky_pairs(n, L, p.Bst, p.pairs_le, p.Bpair, 0));
+        } else {
+            PHF_TRY(build_coulomb_slices(p));
+        }
+        PHF_CUDA(cudaDeviceSynchronize());
         return PHF_OK;
     }
     double *EK = nullptr;
