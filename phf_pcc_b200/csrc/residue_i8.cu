@@ -572,7 +572,8 @@ __global__ void __launch_bounds__(RZ_THREADS, 1)
     uint64_t *empty = full + RZ_STAGES;
     uint64_t *acc_full = empty + RZ_STAGES;   // the tile's MMAs are complete
     uint64_t *acc_empty = acc_full + 1;       // [2] the epilogue has read row half h
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+    uint64_t *drained = acc_empty + 2;        // after a wait gave up: the MMAs issued are complete
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -583,6 +584,7 @@ __global__ void __launch_bounds__(RZ_THREADS, 1)
         }
         rz_mbar_init(acc_full, 1);
         for (int h = 0; h < 2; ++h) rz_mbar_init(&acc_empty[h], RZ_EPI_WARPS);
+        rz_mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -594,6 +596,7 @@ __global__ void __launch_bounds__(RZ_THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     const int ntile = args.mt * args.nt * args.planes;
+    int loads = 0;  // k-blocks whose loads thread 0 has issued
 
     if (warp == 0) {
         if (lane == 0) {  // TMA producer
@@ -614,6 +617,7 @@ __global__ void __launch_bounds__(RZ_THREADS, 1)
                                  : "memory");
                     rz_load(&tmA, &full[sg], dst, kb * RZ_BK, arow, plane);
                     rz_load(&tmB, &full[sg], dst + RZ_OP, kb * RZ_BK, brow, plane);
+                    ++loads;
                     if (++sg == RZ_STAGES) {
                         sg = 0;
                         ph ^= 1u;
@@ -712,6 +716,17 @@ __global__ void __launch_bounds__(RZ_THREADS, 1)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag) {
+        // a wait gave up: MMAs and loads may be in flight, and TMEM and shared memory must outlive them
+        if (warp == 1 && lane == 0) {
+            rz_commit(drained);
+            rz_wait(drained, 0, args.err, 32);
+        }
+        if (threadIdx.x == 0)
+            for (int s = 0; s < min(loads, RZ_STAGES); ++s)  // the last load into each stage
+                rz_wait(&full[s], (uint32_t)((loads - 1 - s) / RZ_STAGES & 1), args.err, 32);
+        __syncthreads();
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
@@ -906,7 +921,7 @@ int rz_map(CUtensorMap *map, const signed char *base, long long kpad, long long 
     return PHF_OK;
 }
 
-constexpr size_t kRzSmem = RZ_STAGES * RZ_STAGE + (2 * RZ_STAGES + 3) * 8 + 8;
+constexpr size_t kRzSmem = RZ_STAGES * RZ_STAGE + (2 * RZ_STAGES + 4) * 8 + 8;
 
 // C_l mod p_l of A rows [a_row0, a_row0 + m) and B rows [b_row0, b_row0 + n) for every plane, contraction
 // length k, into C (rz_pad_rows(m) rows of ldc = rz_pad_rows(n) bytes per plane).
