@@ -395,33 +395,34 @@ size_t rz_scratch(const PlanImpl &p, long long b, RzScratch *out) {
     return tile * (size_t)most + coulomb(32 * most);
 }
 
-// How the Cholesky vectors compare with their transposes (16 x 16 tiles, so that both sides stay in cache): 2 = every
-// B_L is exactly symmetric, 1 = to rounding, 0 = neither (or not finite).  To rounding: no difference above 2 sqrt(n)
-// units in the last place of the largest element of B_L.  Vectors brought to another basis, X^T B X, are sums of n
-// products on either side and differ by 2 (n = 5), 6 (64), 8 (128) and 10 (200) such units; a difference of that size
-// says nothing about the integrals, and the full rows of vectors that are not symmetric cost twice the exchange work.
+// f(B[p][q], B[q][p]) over the pairs of one vector until it returns false (16 x 16 tiles, so that both sides stay in cache)
+template <typename F>
+bool over_pairs(const double *B, int n, F &&f) {
+    const int T = 16;
+    for (int q0 = 0; q0 < n; q0 += T)
+        for (int p0 = 0; p0 <= q0; p0 += T)
+            for (int q = q0; q < std::min(q0 + T, n); ++q)
+                for (int p = p0; p < std::min(p0 + T, q); ++p)
+                    if (!f(B[p + (size_t)n * q], B[q + (size_t)n * p])) return false;
+    return true;
+}
+
+// How the Cholesky vectors compare with their transposes: 2 = every B_L is exactly symmetric, 1 = to rounding,
+// 0 = neither (or not finite).  To rounding: no difference above 2 sqrt(n) units in the last place of the largest
+// element of B_L.  Vectors brought to another basis, X^T B X, are sums of n products on either side and differ by
+// 2 (n = 5), 6 (64), 8 (128) and 10 (200) such units; a difference of that size says nothing about the integrals,
+// and the full rows of vectors that are not symmetric cost twice the exchange work.
 int cholesky_symmetry(const phf_plan_desc *d) {
-    const int n = d->nso / 2, T = 16;
+    const int n = d->nso / 2;
     int level = 2;
     for (int l = 0; l < d->nchol; ++l) {
         const double *B = d->bvec + (size_t)n * n * l;
-        double diff = 0.0;
-        bool exact = true;
-        for (int q0 = 0; q0 < n; q0 += T)
-            for (int p0 = 0; p0 <= q0; p0 += T)
-                for (int q = q0; q < std::min(q0 + T, n); ++q)
-                    for (int p = p0; p < std::min(p0 + T, q); ++p) {
-                        const double a = B[p + (size_t)n * q], b = B[q + (size_t)n * p];
-                        if (a != b) {
-                            exact = false;
-                            if (!(std::fabs(a - b) <= std::numeric_limits<double>::max())) return 0;
-                            diff = std::max(diff, std::fabs(a - b));
-                        }
-                    }
-        if (exact) continue;
+        if (over_pairs(B, n, [](double a, double b) { return a == b; })) continue;
         double mx = 0.0;
         for (size_t e = 0; e < (size_t)n * n; ++e) mx = std::max(mx, std::fabs(B[e]));
-        if (!(diff <= 2.0 * std::sqrt((double)n) * std::numeric_limits<double>::epsilon() * mx)) return 0;
+        const double limit = 2.0 * std::sqrt((double)n) * std::numeric_limits<double>::epsilon() * mx;
+        if (!std::isfinite(limit) || !over_pairs(B, n, [=](double a, double b) { return std::fabs(a - b) <= limit; }))
+            return 0;
         level = 1;
     }
     return level;
