@@ -24,7 +24,8 @@
 // before they are multiplied up, and the parts of a point are added before the weighted sum over the points takes
 // them.  (Weighted sums of each part over the points, antisymmetrised at the end: 1.7 times the error of the
 // sequence as it stands, as a geometric mean over 140 problems with n = 3..6, and up to twelve times; now 0.31.)
-// Assembling t2 point by point in 172 passes over M^4 elements took 28 of the 44 ms of 112 points at M = 32.
+// Assembling t2 point by point in 172 passes over M^4 elements took 28 of the 44 ms of 112 points at M = 32; the
+// whole sequence takes 14.9 now.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -77,6 +78,7 @@ __device__ __forceinline__ void pair_of(long long p, int &e, int &f) {
 
 // out = in antisymmetrised in (a, b) and in (c, d), a point per blockIdx.z: a block takes the planes (c, d) and (d, c)
 // of blockIdx.x's pair and the 32 x 32 tiles (I, J), (J, I) of (a, b), so that every row is read and written whole.
+// Bound: memory, one tensor read and one written (M = 32, 112 points: 3.8 GB in 0.69 ms, 5.5 TB/s).
 constexpr int AT = 32, AT_P = AT + 1;
 __global__ void __launch_bounds__(NT) antisymmetrise_kernel(int M, const zc *__restrict__ in, zc *__restrict__ out) {
     __shared__ zc s1[AT * AT_P], s2[AT * AT_P];
@@ -112,7 +114,8 @@ __global__ void __launch_bounds__(NT) antisymmetrise_kernel(int M, const zc *__r
 // - Y(a,d) V(b,c)]_w for c <= d and the tiles of 32 a and 8 b that reach a <= b.  A warp of the block takes every
 // eighth point (t11(b,c,d,a) through its own 8 x 32 tile of shared memory), the warps' sums are added in order:
 // one warp for all points was a chain of as many load latencies as points.
-// Bound: t11 and a quarter of t12 read once (M = 32, 112 points: 1.9 GB in all).
+// Bound: reading half of t11 and a quarter of t12 once, 128-byte pieces of the transposed half (M = 32, 112 points:
+// 0.90 ms; with the antisymmetrisation 1.6, where tau20's product, the sums over the points and their assembly took 2.4).
 constexpr int PT_B = 8, PT_W = NT / 32;
 __global__ void __launch_bounds__(NT) points_t2_kernel(int M, int b, const zc *__restrict__ t12, const zc *__restrict__ t11,
                                                        const zc *__restrict__ Y, const zc *__restrict__ U,

@@ -552,8 +552,10 @@ __device__ __forceinline__ int rz_cols(int n, int c0) { return min(RZ_TILE, (n -
 
 // C_l mod p_l (one byte, 0 .. p_l) of every plane.  One persistent CTA per SM runs tiles of 256 x 256: two
 // 128 x 256 accumulators fill TMEM, k-blocks of 64 (16 KB of each operand) pass through a seven-stage ring,
-// and each is two MMAs of 128 x 256 x 32 per row half.  At the full MMA rate operands arrive at 64 B per
-// cycle and SM (128 x 256 tiles would need 96) and the MMAs read 94 B per cycle of shared memory.  Epilogue:
+// and each is two MMAs of 128 x 256 x 32 per row half.  At the full MMA rate operands would arrive at 64 B per
+// cycle and SM (at 96 with 128 x 256 tiles).  Counters: tensor pipe 74 % active, operands read from DRAM once, L2 at
+// 60 % of its throughput (n = 101, 312 points: 2496 rows x 5151 x k 5151 x 22, 2.77e15 operations per second);
+// 58 % at k = 2080, where a tile's read-out is a larger part of it.  Epilogue:
 // residues by one high multiplication, 8 warps; a row half is released as soon as it has been read, so the
 // next tile's MMAs wait for half of the read-out (its loads are already in the ring).  A half that lies
 // beyond the last row, and columns beyond the last one rounded up to 32, are not multiplied.  Measured: 3.0e15
