@@ -202,7 +202,8 @@ typedef struct {
                                                  with n > 64 (n <= 64 tensor-core plans slice the densities in the
                                                  fused kernel and run the full rows; 1 is refused there).
                                                  jk_form 1: the FP64 form and the int8 form (n >= 2 with the default
-                                                 slices, n > 64 with slices 1..7).  All but jk_form 3 in FP64 need
+                                                 slices, n > 64 with slices 1..7); no effect in its other
+                                                 forms.  All but jk_form 3 in FP64 need
                                                  Cholesky vectors that are symmetric to rounding, of which
                                                  (B + B^T) / 2 is taken (no difference above 2 sqrt(n) units in the
                                                  last place of a vector's largest element); other vectors run the
