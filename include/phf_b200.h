@@ -338,7 +338,7 @@ int phf_int8_wide_mma(int on);
 int phf_int8_fock_product(int on);
 /* The one-shot calls (phf_buildhsg, phf_buildhsg_chol, phf_localg, phf_buildsc, phf_pbarhbarolap) keep the device
    memory they used for the next one: at most 16 GiB and at most half of what is free when a call ends.  A
-   cudaMalloc of the same process that would fail gets it; this returns the current device's to the driver, for
+   cudaMalloc of the same process that would fail gets it; this returns the current device's to the CUDA driver, for
    other processes and for what counts the free memory. */
 void phf_release_memory(void);
 /* Library version string. */

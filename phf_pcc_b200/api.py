@@ -195,7 +195,7 @@ def buildsc(c0, c1, c2, nocc, ngrid, qj, r1, r2, rpg, rk, roota, rootb, rooty, w
 
 
 def release_memory() -> None:
-    """Return the device memory that one-shot calls keep for the next one (at most 16 GiB) to the driver, for
+    """Return the device memory that one-shot calls keep for the next one (at most 16 GiB) to the CUDA driver, for
     other processes (a cudaMalloc of this process that would fail gets it without this call)."""
     _lib.load().phf_release_memory()
 

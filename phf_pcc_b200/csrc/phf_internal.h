@@ -21,9 +21,9 @@ struct DevBuf {
 // Device memory of calls that allocate and free within themselves (one-shot buildhsg, localg, BuildSC, the
 // projected-CC kernel): a stream-ordered pool per device, on the legacy default stream, which is where those
 // calls run.  It keeps freed memory for the next call, at most 16 GiB and at most half of what is free on the
-// device when a call ends (pool_trim).  The driver takes it back for a cudaMalloc of this process that
+// device when a call ends (pool_trim).  The CUDA driver takes it back for a cudaMalloc of this process that
 // would fail otherwise (a plan's, another allocator's), pool_alloc gives it back before it tries once more, and
-// phf_release_memory does so for other processes.  Safe for several threads: the pool is the driver's, and every
+// phf_release_memory does so for other processes.  Safe for several threads: the pool is the CUDA driver's, and every
 // use is ordered on the one stream.
 // (With cudaMalloc and cudaFree in every call: projected-CC kernel, M = 40, 92 ms against 50; BuildSC, M = 32, 49
 // against 20, ten of them the division by the overlap on the host.)
